@@ -1515,11 +1515,68 @@ __global__ void k_rec_place_min(const Rec* __restrict__ in, const uint32_t* __re
   if (lane_id() == 0 && hub_min != kInf64) red_min(&minval[hub], hub_min);
 }
 
-// D at `count` pseudo-random vertices (for picking the largest component).
-__global__ void k_sample_labels(uint32_t n, const uint32_t* __restrict__ D, uint64_t seed,
-                                uint32_t count, uint32_t* out) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-    out[i] = D[__umul64hi(mix64(seed ^ (0x9e3779b97f4a7c15ull * (i + 1))), n)];
+// One CTA draws kSampleCount values (value(i), i < kSampleCount) and leaves
+// them in `out` in ascending order; the host reads quantiles and run lengths
+// from it.  A bitonic network over the elements 4t + k of thread t: steps of
+// 1 and 2 stay in the thread, 4 to 64 in the warp (shuffles), and only the 15
+// steps of 128 and more go through shared memory and barriers (a network with
+// all 78 steps there took 35 us a sample against 26 us now, reads and all; the
+// host's sort of the same sample about 60 us).
+constexpr uint32_t kSampleCount = 4096;
+constexpr int kSampleBlock = 1024;
+template <typename Value>
+__device__ __forceinline__ void sample_sorted(Value value, uint32_t* __restrict__ out) {
+  __shared__ __align__(16) uint32_t s[kSampleCount];
+  constexpr int kPer = kSampleCount / kSampleBlock;
+  static_assert(kPer == 4, "the network's thread-local steps are 1 and 2");
+  const uint32_t i0 = threadIdx.x * kPer;
+  uint32_t v[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) v[k] = value(i0 + k);
+  // element i takes the smaller of the pair (i, i ^ step) when bit `step` of
+  // i is 0 and its block of `size` sorts upwards, or both are the other way
+  auto pick = [](uint32_t i, uint32_t size, uint32_t step, uint32_t mine, uint32_t other) {
+    return ((i & step) == 0) == ((i & size) == 0) ? min(mine, other) : max(mine, other);
+  };
+  for (uint32_t size = 2; size <= kSampleCount; size <<= 1) {
+    for (uint32_t step = size >> 1; step >= 128; step >>= 1) {
+      __syncthreads();
+      *reinterpret_cast<uint4*>(s + i0) = make_uint4(v[0], v[1], v[2], v[3]);
+      __syncthreads();
+      const uint4 o = *reinterpret_cast<const uint4*>(s + (i0 ^ step));
+      v[0] = pick(i0, size, step, v[0], o.x);
+      v[1] = pick(i0 + 1, size, step, v[1], o.y);
+      v[2] = pick(i0 + 2, size, step, v[2], o.z);
+      v[3] = pick(i0 + 3, size, step, v[3], o.w);
+    }
+    for (uint32_t step = min(size >> 1, 64u); step >= 4; step >>= 1) {
+#pragma unroll
+      for (int k = 0; k < kPer; ++k)
+        v[k] = pick(i0 + k, size, step, v[k], __shfl_xor_sync(kFull, v[k], step / kPer));
+    }
+#pragma unroll
+    for (uint32_t step = 2; step >= 1; step >>= 1) {
+      if (step >= size) continue;
+      uint32_t x[kPer];
+#pragma unroll
+      for (uint32_t k = 0; k < kPer; ++k) x[k] = pick(i0 + k, size, step, v[k], v[k ^ step]);
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) v[k] = x[k];
+    }
+  }
+  *reinterpret_cast<uint4*>(out + i0) = make_uint4(v[0], v[1], v[2], v[3]);
+}
+
+// D at kSampleCount pseudo-random vertices, sorted (for picking the largest
+// component).
+__global__ void __launch_bounds__(kSampleBlock)
+    k_sample_labels(uint32_t n, const uint32_t* __restrict__ D, uint64_t seed,
+                    uint32_t* __restrict__ out) {
+  sample_sorted(
+      [&](uint32_t i) {
+        return D[__umul64hi(mix64(seed ^ (0x9e3779b97f4a7c15ull * (i + 1))), n)];
+      },
+      out);
 }
 
 // Shortcut every original vertex to its new representative and compute its
@@ -1550,6 +1607,20 @@ __global__ void k_iota(uint32_t n, uint32_t* __restrict__ a) {
   for (uint64_t x = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; x < n;
        x += static_cast<uint64_t>(gridDim.x) * blockDim.x)
     a[x] = static_cast<uint32_t>(x);
+}
+
+// Start of a solve: minima at infinity and, when labels are needed (several
+// contractions), the identity in the representative and label arrays.
+__global__ void k_init_vertices(uint32_t n, uint64_t* __restrict__ minval,
+                                uint32_t* __restrict__ P, uint32_t* __restrict__ V,
+                                uint32_t* __restrict__ D) {
+  for (uint64_t x = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; x < n;
+       x += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+    minval[x] = kInf64;
+    V[x] = static_cast<uint32_t>(x);
+    P[x] = static_cast<uint32_t>(x);
+    D[x] = static_cast<uint32_t>(x);
+  }
 }
 
 __global__ void k_fill64(uint64_t n, uint64_t* __restrict__ a, uint64_t v) {
@@ -1611,27 +1682,27 @@ __global__ void k_mark_forest(uint64_t k, const uint32_t* __restrict__ msf,
   }
 }
 
-// Weight samples for pivot selection: sample i reads the weight of the input
-// entry at hi64(mix64(seed + i) * m).  Both copies of an undirected edge
-// carry its weight, so sampling the directed list samples edge weights.
-__global__ void k_sample_weights(const uint32_t* __restrict__ in_words, uint64_t m,
-                                 uint64_t seed, uint32_t count, uint32_t* out) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count;
-       i += gridDim.x * blockDim.x) {
-    const uint64_t pos = __umul64hi(mix64(seed + i), m);
-    out[i] = in_words[pos * 3 + 2];
-  }
+// Weight samples for pivot selection, sorted: sample i is the weight of the
+// input entry at hi64(mix64(seed + i) * m).  Both copies of an undirected
+// edge carry its weight, so sampling the directed list samples edge weights.
+__global__ void __launch_bounds__(kSampleBlock)
+    k_sample_weights(const uint32_t* __restrict__ in_words, uint64_t m, uint64_t seed,
+                     uint32_t* __restrict__ out) {
+  sample_sorted(
+      [&](uint32_t i) { return in_words[__umul64hi(mix64(seed + i), m) * 3 + 2]; }, out);
 }
 
 // Same over a segmented list; prefix[s] = records in segments < s.
-__global__ void k_sample_weights_seg(SegIn in, const uint64_t* __restrict__ prefix, uint64_t m,
-                                     uint64_t seed, uint32_t count, uint32_t* out) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count;
-       i += gridDim.x * blockDim.x) {
-    const uint64_t x = __umul64hi(mix64(seed + i), m);
-    const uint32_t sg = seg_find(prefix, in.nseg, x);
-    out[i] = in.base[static_cast<uint64_t>(sg) * in.cap + (x - prefix[sg])].w;
-  }
+__global__ void __launch_bounds__(kSampleBlock)
+    k_sample_weights_seg(SegIn in, const uint64_t* __restrict__ prefix, uint64_t m,
+                         uint64_t seed, uint32_t* __restrict__ out) {
+  sample_sorted(
+      [&](uint32_t i) {
+        const uint64_t x = __umul64hi(mix64(seed + i), m);
+        const uint32_t sg = seg_find(prefix, in.nseg, x);
+        return in.base[static_cast<uint64_t>(sg) * in.cap + (x - prefix[sg])].w;
+      },
+      out);
 }
 
 }  // namespace kamsta

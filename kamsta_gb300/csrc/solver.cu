@@ -107,7 +107,7 @@ static inline uint32_t ceil_div(uint64_t a, uint64_t b) {
   return static_cast<uint32_t>((a + b - 1) / b);
 }
 
-constexpr uint32_t kSamples = 4096;
+static_assert(kSampleCount == kSampleCap, "the context holds one sample");
 // Round passes over at most this many vertices use 4-record tiles.
 constexpr uint32_t kWideRoundN = 1u << 16;
 // Largest next-round label count whose minima a list pass keeps per CTA in
@@ -199,7 +199,8 @@ class Solve {
   bool use_big_ = false;
   uint32_t big_label_ = 0;
   std::vector<uint32_t> plan_classes();
-  kamsta_status sample_weights(const SegList* L, uint32_t count, std::vector<uint32_t>* out);
+  kamsta_status sample_weights(const SegList* L, std::vector<uint32_t>* out);
+  kamsta_status fetch_samples(std::vector<uint32_t>* out);
   kamsta_status filter_rec(SegList* L, bool own, bool stop, int depth);
   kamsta_status run_boruvka();
   kamsta_status run_filter_boruvka();
@@ -846,7 +847,15 @@ kamsta_status Solve::rounds(SegList* L, bool own) {
 // ---------------------------------------------------------------------------
 // sampling and planning
 
-kamsta_status Solve::sample_weights(const SegList* L, uint32_t count, std::vector<uint32_t>* out) {
+kamsta_status Solve::fetch_samples(std::vector<uint32_t>* out) {
+  CU_TRY(cudaMemcpyAsync(ctx_->h_samples, samples_, kSampleCount * sizeof(uint32_t),
+                         cudaMemcpyDeviceToHost, st_));
+  CU_TRY(cudaStreamSynchronize(st_));
+  out->assign(ctx_->h_samples, ctx_->h_samples + kSampleCount);
+  return KAMSTA_OK;
+}
+
+kamsta_status Solve::sample_weights(const SegList* L, std::vector<uint32_t>* out) {
   out->clear();
   uint64_t m = L ? L->total : md_;
   if (!L && !input_complete_) {  // only the first piece of the input is there yet
@@ -854,26 +863,20 @@ kamsta_status Solve::sample_weights(const SegList* L, uint32_t count, std::vecto
     m = io_->piece_end[0];
   }
   if (m == 0) return KAMSTA_OK;
-  count = std::min<uint32_t>(count, kSamples);
-  const int g = grid_for(count);
   const int tp = tick();
   if (L) {
     std::vector<uint64_t> pre(L->nseg + 1, 0);
     for (uint32_t s = 0; s < L->nseg; ++s) pre[s + 1] = pre[s] + L->h_count[s];
     CU_TRY(cudaMemcpyAsync(prefix_, pre.data(), sizeof(uint64_t) * (L->nseg + 1),
                            cudaMemcpyHostToDevice, st_));
-    k_sample_weights_seg<<<g, kBlock, 0, st_>>>(L->in(), prefix_, m, cfg_.seed, count, samples_);
+    k_sample_weights_seg<<<1, kSampleBlock, 0, st_>>>(L->in(), prefix_, m, cfg_.seed, samples_);
   } else {
-    k_sample_weights<<<g, kBlock, 0, st_>>>(in_, m, cfg_.seed, count, samples_);
+    k_sample_weights<<<1, kSampleBlock, 0, st_>>>(in_, m, cfg_.seed, samples_);
   }
   tock(KAMSTA_PHASE_PLAN, tp);
-  account(KAMSTA_PHASE_PLAN, uint64_t(count) * 8, 1);
-  out->resize(count);
-  CU_TRY(cudaMemcpyAsync(out->data(), samples_, count * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                         st_));
-  CU_TRY(cudaStreamSynchronize(st_));
+  account(KAMSTA_PHASE_PLAN, uint64_t(kSampleCount) * 8, 1);
+  KS_TRY(fetch_samples(out));
   resolve();
-  std::sort(out->begin(), out->end());
   return KAMSTA_OK;
 }
 
@@ -885,7 +888,7 @@ std::vector<uint32_t> Solve::plan_classes() {
   std::vector<uint32_t> thr;
   if (cfg_.local_preprocessing == KAMSTA_NO_PREPROCESSING) return thr;
   std::vector<uint32_t>& s = samples_host_;
-  if (sample_weights(nullptr, kSamples, &s) != KAMSTA_OK) return thr;
+  if (sample_weights(nullptr, &s) != KAMSTA_OK) return thr;
   double m_est = static_cast<double>(md_) / 2.0;
   const double nv = static_cast<double>(n_);
   size_t len = s.size();
@@ -923,14 +926,10 @@ static double sample_share(const std::vector<uint32_t>& s, uint32_t lo, uint32_t
 kamsta_status Solve::pick_big(uint32_t* label, bool* use) {
   *use = false;
   if (n_ < (1u << 16) || nreps_ <= 1) return KAMSTA_OK;
-  const uint32_t count = kSamples;
-  k_sample_labels<<<grid_for(count), kBlock, 0, st_>>>(n_, D_, cfg_.seed ^ launches_, count,
-                                                       samples_);
-  std::vector<uint32_t> h(count);
-  CU_TRY(cudaMemcpyAsync(h.data(), samples_, count * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                         st_));
-  CU_TRY(cudaStreamSynchronize(st_));
-  std::sort(h.begin(), h.end());
+  const uint32_t count = kSampleCount;
+  k_sample_labels<<<1, kSampleBlock, 0, st_>>>(n_, D_, cfg_.seed ^ launches_, samples_);
+  std::vector<uint32_t> h;
+  KS_TRY(fetch_samples(&h));
   uint32_t best = 0, best_len = 0;
   for (size_t i = 0; i < h.size();) {
     size_t j = i;
@@ -1064,7 +1063,6 @@ kamsta_status Solve::run_boruvka() {
   const uint32_t wmax0 = K == 0 ? 0xffffffffu : b[nmat - 1];
   // first pass: classes 0..nmat-1, class 0 with identity labels and the
   // round-0 minimum fused in
-  fill_inf(minA_, n_);
   SegList* C[kMaxOut] = {new_list(), new_list(), new_list()};
   double frac[kMaxOut] = {1.0, 1.0, 1.0};
   if (K > 0)
@@ -1134,7 +1132,7 @@ kamsta_status Solve::filter_rec(SegList* L, bool own, bool stop, int depth) {
     return KAMSTA_OK;
   }
   std::vector<uint32_t> s;
-  KS_TRY(sample_weights(L, kSamples, &s));
+  KS_TRY(sample_weights(L, &s));
   const uint32_t pivot = s[s.size() / 2];
   SegList* light = new_list();
   SegList* heavy = new_list();
@@ -1242,10 +1240,8 @@ kamsta_status Solve::run(Algo algo, kamsta_wedge* d_out, SolveOut* out) {
     std::vector<uint32_t> thr_desc = plan_classes();
     bounds_.assign(thr_desc.rbegin(), thr_desc.rend());
   }
-  k_iota<<<grid_for(n_), kBlock, 0, st_>>>(n_, P_);
-  k_iota<<<grid_for(n_), kBlock, 0, st_>>>(n_, V_);
-  k_iota<<<grid_for(n_), kBlock, 0, st_>>>(n_, D_);
-  account(KAMSTA_PHASE_FINALIZE, uint64_t(n_) * 12, 3);
+  k_init_vertices<<<grid_for(n_), kBlock, 0, st_>>>(n_, minA_, P_, V_, D_);
+  account(KAMSTA_PHASE_FINALIZE, uint64_t(n_) * 20, 1);
   nreps_ = n_;
   msf_count_ = 0;
   d_out_ = d_out;

@@ -45,6 +45,7 @@ static_assert(sizeof(DevCounters) == 128, "counter block size");
 enum CounterSlot : int { kCVertex = 0, kCEdge = 1, kCRep = 2, kCMisc = 3, kCSlots = 4 };
 constexpr uint32_t kSampleCap = 4096;
 constexpr int kTimerEvents = 64;
+constexpr size_t kHostState = 1024;  // bytes of kamsta_ctx::h_state
 constexpr int kInputPieces = 16;  // host input copied in this many pieces
 
 }  // namespace kamsta
@@ -67,6 +68,8 @@ struct kamsta_ctx {
   uint32_t* d_err = nullptr;
   kamsta::DevCounters* h_counters = nullptr;  // pinned mirror
   uint32_t* h_err = nullptr;
+  uint32_t* h_samples = nullptr;  // pinned: the sorted samples
+  void* h_state = nullptr;        // pinned: head of the cooperative solve's state
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t tev[kamsta::kTimerEvents] = {};  // per-phase timing events
   kamsta::Arena io;      // host-buffer entry points: device copies of in/out
