@@ -21,8 +21,10 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 
 #include "kernels.cuh"
+#include "rounds_coop.cuh"
 #include "solver.cuh"
 #include "sort_gen.cuh"
 
@@ -144,6 +146,7 @@ class Solve {
       free_list(L);
       delete L;
     }
+    if (coop_mem_) cudaFreeAsync(coop_mem_, st_);
   }
 
   kamsta_status run(Algo algo, kamsta_wedge* d_out, SolveOut* out);
@@ -178,7 +181,7 @@ class Solve {
   template <int NOUT>
   kamsta_status pass(int phase, const SegList* src, const uint32_t* map, uint32_t wmin,
                      uint32_t wmax, const uint32_t* thr, SegList* const* outs, const double* frac,
-                     uint64_t* minval, uint64_t minval_n, bool validate);
+                     uint64_t* minval, uint64_t minval_n, bool validate, bool fetch = true);
   // Boruvka rounds on list L (dense labels in [0, nreps_)); minA_ holds the
   // round-0 minima.  Frees L if `own` is set.
   kamsta_status rounds(SegList* L, bool own);
@@ -203,6 +206,21 @@ class Solve {
   kamsta_status fetch_samples(std::vector<uint32_t>* out);
   kamsta_status filter_rec(SegList* L, bool own, bool stop, int depth);
   kamsta_status run_boruvka();
+  // The first pass; with fetch = false its counts stay on the device.
+  kamsta_status first_pass(SegList** C, int nmat, bool fetch);
+  // ---- cooperative rounds (rounds_coop.cuh)
+  // Whole solve in one launch per weight class without host reads; *done is
+  // false when the solve has to run by host-driven rounds instead.
+  bool coop_fits() const;
+  kamsta_status run_coop(bool* done);
+  kamsta_status coop_launch(const SegList* L, uint64_t md, uint32_t wmin, uint32_t wmax,
+                            bool prologue, bool finalize, bool emit);
+  kamsta_status coop_reset();
+  kamsta_status coop_fetch();
+  uint32_t coop_grid_ = 0, coop_launches_ = 0;
+  uint64_t coop_cap_ = 0;     // records per segment of the two buffers
+  Rec* coop_buf_[2] = {nullptr, nullptr};
+  bool coop_done_ = false;    // the solve's forest is written
   kamsta_status run_filter_boruvka();
   // ---- debugging (KAMSTA_DEBUG_CHECKS=1): host-side invariant checks
   kamsta_status debug_list(const char* where, const SegList& L, uint64_t nlabels);
@@ -272,6 +290,10 @@ class Solve {
   uint64_t *minA_ = nullptr, *minB_ = nullptr, *prefix_ = nullptr;
   uint32_t* cta_counts_ = nullptr;  // per-CTA counts of the vertex scans
   uint32_t* big_ = nullptr;         // membership bitmap of the largest component
+  void* coop_mem_ = nullptr;
+  coop::State* coop_state_ = nullptr;
+  uint64_t* coop_tiny_ = nullptr;
+  uint32_t* coop_cnt_ = nullptr;
   uint32_t nreps_ = 0;
   uint64_t msf_count_ = 0;
   bool input_complete_ = true;  // every later input reader is ordered after the last piece
@@ -456,7 +478,7 @@ template <int NOUT>
 kamsta_status Solve::pass(int phase, const SegList* src, const uint32_t* map, uint32_t wmin,
                           uint32_t wmax, const uint32_t* thr, SegList* const* outs,
                           const double* frac, uint64_t* minval, uint64_t minval_n,
-                          bool validate) {
+                          bool validate, bool fetch) {
   const bool dir = src == nullptr;
   const uint64_t total = dir ? md_ : src->total;
   const int items = (map != nullptr && dir_items_ == 8) ? kMappedDirItems : dir_items_;
@@ -573,6 +595,10 @@ kamsta_status Solve::pass(int phase, const SegList* src, const uint32_t* map, ui
       k_pass_seg<NOUT, 8><<<G, kBlock, dyn, st_>>>(src->in(), a);
     tock(phase, t0);
     CU_TRY(cudaGetLastError());
+    if (!fetch) {  // the counts stay on the device (cooperative rounds)
+      account(phase, total * (dir ? 12 : sizeof(Rec)), 1);
+      return KAMSTA_OK;
+    }
     for (int c = 0; c < NOUT; ++c)
       CU_TRY(cudaMemcpyAsync(outs[c]->h_count.data(), outs[c]->d_count, sizeof(uint32_t) * G,
                              cudaMemcpyDeviceToHost, st_));
@@ -1056,14 +1082,213 @@ kamsta_status Solve::contract(const SegList* L, uint32_t wmin, uint32_t wmax, do
   return rounds(E, true);
 }
 
-kamsta_status Solve::run_boruvka() {
-  const std::vector<uint32_t>& b = bounds_;  // ascending class bounds
+// ---------------------------------------------------------------------------
+// cooperative rounds
+
+// Cooperative launches of one process run one after another on a device:
+// each waits for the event of the one before, so that two grids whose CTAs
+// wait for one another are never on the device together, whatever streams
+// and threads they come from.
+namespace {
+struct CoopOrder {
+  std::mutex mu;
+  cudaEvent_t ev = nullptr;
+};
+constexpr int kCoopDevices = 64;
+CoopOrder g_coop_order[kCoopDevices];
+
+cudaError_t launch_in_order(int dev, const void* f, uint32_t grid, uint32_t block, size_t smem,
+                            void** args, cudaStream_t st) {
+  if (dev < 0 || dev >= kCoopDevices) return cudaErrorInvalidDevice;
+  CoopOrder& o = g_coop_order[dev];
+  std::lock_guard<std::mutex> lock(o.mu);
+  cudaError_t e = cudaSuccess;
+  if (!o.ev) e = cudaEventCreateWithFlags(&o.ev, cudaEventDisableTiming);
+  else e = cudaStreamWaitEvent(st, o.ev, 0);
+  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(f, dim3(grid), dim3(block), args, smem, st);
+  if (e == cudaSuccess) e = cudaEventRecord(o.ev, st);
+  return e;
+}
+}  // namespace
+
+// Inputs of fewer entries are solved by cooperative rounds: their host-driven
+// rounds spend more on launches and host reads than on the edges.  Average
+// degree 16, host-driven against cooperative: 2^16 entries 457 / 136 us, 2^20
+// 575 / 183, 2^24 1272 / 859 (G(n,m), no preprocessing) and 1383 / 486 (RGG,
+// local preprocessing).  From 2^25 on the heaviest class is better contracted
+// by row scans than by the stream used here (2^26: 400 MB of reads).
+constexpr uint64_t kCoopMaxMd = (1ull << 25) - 1;
+
+bool Solve::coop_fits() const {
+  // per-round traces, dedupe between rounds and the debug checks are the
+  // host-driven rounds' alone
+  if (debug_ || (cfg_.flags & (KAMSTA_FLAG_TRACE | KAMSTA_FLAG_DEDUPE_ALWAYS))) return false;
+  if (cfg_.dedupe_ratio && !(cfg_.flags & KAMSTA_FLAG_DEDUPE_NEVER)) return false;
+  return n_ >= 2 && n_ < kRootTag && md_ <= kCoopMaxMd &&
+         bounds_.size() + 1 <= coop::kMaxLaunch;
+}
+
+// The state, the tiny rounds' minima and the buffers' counts come from the
+// pool, not the fixed arena: a memory limit that leaves no room for them
+// still solves by host-driven rounds.
+kamsta_status Solve::coop_reset() {
+  coop_launches_ = 0;
+  if (!coop_mem_) {
+    const size_t sb = round_up(sizeof(coop::State), 256);
+    const size_t tb = sizeof(uint64_t) * 3 * coop::kTinyN;
+    CU_TRY(ctx_alloc(ctx_, &coop_mem_, sb + tb + sizeof(uint32_t) * 2 * kMaxSeg, st_));
+    char* m = static_cast<char*>(coop_mem_);
+    coop_state_ = reinterpret_cast<coop::State*>(m);
+    coop_tiny_ = reinterpret_cast<uint64_t*>(m + sb);
+    coop_cnt_ = reinterpret_cast<uint32_t*>(m + sb + tb);
+  }
+  CU_TRY(cudaMemsetAsync(coop_state_, 0, sizeof(coop::State), st_));
+  return KAMSTA_OK;
+}
+
+kamsta_status Solve::coop_launch(const SegList* L, uint64_t md, uint32_t wmin, uint32_t wmax,
+                                 bool prologue, bool finalize, bool emit) {
+  coop::Args a{};
+  if (L) {
+    a.src = L->base;
+    a.src_count = L->d_count;
+    a.src_cap = L->cap;
+    a.src_nseg = L->nseg;
+  }
+  a.in = in_;
+  a.md = static_cast<uint32_t>(md);
+  a.wmin = wmin;
+  a.wmax = wmax;
+  a.prologue = prologue ? 1u : 0u;
+  for (int k = 0; k < 2; ++k) {
+    a.buf[k] = coop_buf_[k];
+    a.cnt[k] = coop_cnt_ + k * kMaxSeg;
+  }
+  a.cap = static_cast<uint32_t>(coop_cap_);
+  a.n = n_;
+  a.first = coop_launches_ == 0 ? 1u : 0u;
+  a.direct = direct_emit_ && coop_launches_ == 0 ? 1u : 0u;
+  a.finalize = finalize ? 1u : 0u;
+  a.emit = !emit ? coop::Emit::kNone : forest_bits_ ? coop::Emit::kBits : coop::Emit::kEdges;
+  a.P = P_;
+  a.D = D_;
+  a.V = V_;
+  a.Vn = Vn_;
+  a.dense_of = dense_of_;
+  a.parent = parent_;
+  a.msfoid = msfoid_;
+  a.msf = msf_;
+  a.R = Rbuf_;
+  a.orig = Obuf_;
+  a.minA = minA_;
+  a.minB = minB_;
+  a.tiny = coop_tiny_;
+  a.vcnt = cta_counts_;
+  a.out = reinterpret_cast<uint32_t*>(d_out_);
+  a.bits = forest_bits_;
+  a.launch = coop_launches_;
+  a.st = coop_state_;
+  a.pass_err = ctx_->d_err;
+  a.err = &coop_state_->errs[coop_launches_];
+  void* args[] = {&a};
+  const int t0 = tick();
+  CU_TRY(launch_in_order(ctx_->device, reinterpret_cast<const void*>(&coop::k_rounds), coop_grid_,
+                         coop::kThreads, sizeof(coop::Shared), args, st_));
+  tock(KAMSTA_PHASE_ROUND_EDGES, t0);
+  ++coop_launches_;
+  return KAMSTA_OK;
+}
+
+kamsta_status Solve::coop_fetch() {
+  static_assert(coop::kStateHead <= kHostState, "pinned mirror of the state's head");
+  CU_TRY(cudaMemcpyAsync(ctx_->h_state, coop_state_, coop::kStateHead, cudaMemcpyDeviceToHost,
+                         st_));
+  return fetch_counters();
+}
+
+kamsta_status Solve::run_coop(bool* done) {
+  *done = false;
+  const std::vector<uint32_t>& b = bounds_;
   const int K = static_cast<int>(b.size());
   const int nmat = std::max(1, std::min(K, kMaxOut));
+  SegList* C[kMaxOut] = {new_list(), new_list(), new_list()};
+  // one CTA per SM; small graphs take fewer, so that their barriers are short
+  const uint64_t work = md_ / 2 + n_;
+  const uint64_t step = uint64_t(coop::kThreads) * coop::kItems;
+  coop_grid_ = static_cast<uint32_t>(
+      std::max<uint64_t>(1, std::min<uint64_t>(std::min(sms_, kMaxSeg / coop::kGroups),
+                                               (work + step - 1) / step)));
+  const kamsta_status s = [&]() -> kamsta_status {
+    KS_TRY(first_pass(C, nmat, false));
+    // a list holds at most one copy of each edge; the classes left in the
+    // input leave at most their share of a group's chunk of it
+    const uint32_t nq = coop_grid_ * coop::kGroups;
+    uint64_t cap = 0;
+    for (int c = 0; c < nmat; ++c)
+      cap = std::max(cap, (std::min<uint64_t>(md_ / 2 + 1, C[c]->nseg * C[c]->cap) + nq - 1) / nq);
+    for (int c = nmat; c <= K; ++c) {
+      const double f = std::min(1.0, sample_share(samples_host_, b[c - 1] + 1,
+                                                  c < K ? b[c] : 0xffffffffu));
+      const uint64_t chunk = (md_ + nq - 1) / nq;
+      const double est = f * chunk * 1.1 + 6.0 * std::sqrt(f * chunk) + step;
+      cap = std::max(cap, std::min<uint64_t>(chunk, static_cast<uint64_t>(est)));
+    }
+    coop_cap_ = cap;
+    SegList* B0 = new_list();
+    KS_TRY(alloc_list(B0, nq, cap));
+    coop_buf_[0] = B0->base;
+    if (K == 0 && C[0]->nseg * C[0]->cap >= nq * cap) {
+      coop_buf_[1] = C[0]->base;  // read for the last time before it is written
+    } else {
+      SegList* B1 = new_list();
+      KS_TRY(alloc_list(B1, nq, cap));
+      coop_buf_[1] = B1->base;
+    }
+    KS_TRY(coop_reset());
+    for (int c = 0; c <= std::max(K, nmat - 1); ++c) {
+      const bool last = c == std::max(K, nmat - 1);
+      const uint32_t lo = c < nmat ? 0u : b[c - 1] + 1;
+      const uint32_t hi = c < nmat || c >= K ? 0xffffffffu : b[c];
+      KS_TRY(coop_launch(c < nmat ? C[c] : nullptr, md_, lo, hi, c > 0, !last, last));
+    }
+    return coop_fetch();
+  }();
+  direct_emit_ = false;
+  for (SegList* L : owned_) free_list(L);
+  coop_buf_[0] = coop_buf_[1] = nullptr;
+  const coop::State& h = *static_cast<const coop::State*>(ctx_->h_state);
+  uint32_t err = 0;
+  if (s == KAMSTA_OK)
+    for (uint32_t k = 0; k < coop_launches_; ++k) err |= h.errs[k];
+  // rejected input is rejected; anything else (no memory for the buffers, a
+  // list larger than the sample promised) is solved by host-driven rounds
+  if (s == KAMSTA_E_INPUT) return s;
+  if (s != KAMSTA_OK || err != 0) {
+    cudaGetLastError();
+    k_init_vertices<<<grid_for(n_), kBlock, 0, st_>>>(n_, minA_, P_, V_, D_);
+    CU_TRY(cudaMemsetAsync(dweight_, 0, sizeof(unsigned long long), st_));
+    CU_TRY(cudaMemsetAsync(ctx_->d_err, 0, sizeof(uint32_t), st_));
+    if (forest_bits_)
+      CU_TRY(cudaMemsetAsync(forest_bits_, 0, sizeof(uint32_t) * ((md_ + 31) / 32), st_));
+    return KAMSTA_OK;
+  }
+  msf_count_ = h.msf_count;
+  rounds_ += h.rounds;
+  levels_ += h.levels;
+  // per record: read, two labels, written again, two minima; per vertex of a
+  // round: minimum, record, partner, parent, label and compaction
+  account(KAMSTA_PHASE_ROUND_EDGES, h.sum_m * 56 + h.sum_n * 60, coop_launches_);
+  coop_done_ = true;
+  *done = true;
+  return KAMSTA_OK;
+}
+
+kamsta_status Solve::first_pass(SegList** C, int nmat, bool fetch) {
+  const std::vector<uint32_t>& b = bounds_;  // ascending class bounds
+  const int K = static_cast<int>(b.size());
   const uint32_t wmax0 = K == 0 ? 0xffffffffu : b[nmat - 1];
   // first pass: classes 0..nmat-1, class 0 with identity labels and the
   // round-0 minimum fused in
-  SegList* C[kMaxOut] = {new_list(), new_list(), new_list()};
   double frac[kMaxOut] = {1.0, 1.0, 1.0};
   if (K > 0)
     for (int c = 0; c < nmat; ++c)
@@ -1072,20 +1297,30 @@ kamsta_status Solve::run_boruvka() {
   // direct emission: the first pass keys the round-0 minima by partner and
   // the first round writes its forest edges to the output
   direct_emit_ = d_out_ != nullptr && forest_bits_ == nullptr && n_ >= 2 && msf_count_ == 0;
+  const int ph = KAMSTA_PHASE_FIRST_PASS;
   switch (nmat) {
     case 1:
-      KS_TRY(pass<1>(KAMSTA_PHASE_FIRST_PASS, nullptr, nullptr, 0, wmax0, nullptr, C, frac, minA_,
-                     n_, validate));
-      break;
+      return pass<1>(ph, nullptr, nullptr, 0, wmax0, nullptr, C, frac, minA_, n_, validate, fetch);
     case 2:
-      KS_TRY(pass<2>(KAMSTA_PHASE_FIRST_PASS, nullptr, nullptr, 0, wmax0, b.data(), C, frac,
-                     minA_, n_, validate));
-      break;
+      return pass<2>(ph, nullptr, nullptr, 0, wmax0, b.data(), C, frac, minA_, n_, validate,
+                     fetch);
     default:
-      KS_TRY(pass<3>(KAMSTA_PHASE_FIRST_PASS, nullptr, nullptr, 0, wmax0, b.data(), C, frac,
-                     minA_, n_, validate));
-      break;
+      return pass<3>(ph, nullptr, nullptr, 0, wmax0, b.data(), C, frac, minA_, n_, validate,
+                     fetch);
   }
+}
+
+kamsta_status Solve::run_boruvka() {
+  if (coop_fits()) {
+    bool done = false;
+    KS_TRY(run_coop(&done));
+    if (done) return KAMSTA_OK;
+  }
+  const std::vector<uint32_t>& b = bounds_;  // ascending class bounds
+  const int K = static_cast<int>(b.size());
+  const int nmat = std::max(1, std::min(K, kMaxOut));
+  SegList* C[kMaxOut] = {new_list(), new_list(), new_list()};
+  KS_TRY(first_pass(C, nmat, true));
   for (int c = 0; c < nmat; ++c) KS_TRY(debug_list("after first pass", *C[c], n_));
   // the last contraction skips the final label update (nothing reads it)
   const int steps = nmat + std::max(0, K - nmat + 1);
@@ -1183,6 +1418,8 @@ kamsta_status Solve::run(Algo algo, kamsta_wedge* d_out, SolveOut* out) {
     const char* dbg = std::getenv("KAMSTA_DEBUG_CHECKS");
     debug_ = dbg && dbg[0] == '1';
   }
+  CU_TRY(cudaFuncSetAttribute(coop::k_rounds, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              static_cast<int>(sizeof(coop::Shared))));
   {  // per device context; cheap
     const int dr = static_cast<int>(rec_dyn_smem(8)), dr4 = static_cast<int>(rec_dyn_smem(4));
     const int d8 = static_cast<int>(dir_dyn_smem(8)), d12 = static_cast<int>(dir_dyn_smem(12)),
@@ -1249,9 +1486,10 @@ kamsta_status Solve::run(Algo algo, kamsta_wedge* d_out, SolveOut* out) {
   CU_TRY(cudaMemsetAsync(dweight_, 0, sizeof(unsigned long long), st_));
   CU_TRY(cudaMemsetAsync(ctx_->d_err, 0, sizeof(uint32_t), st_));
   KS_TRY(algo == Algo::kBoruvka ? run_boruvka() : run_filter_boruvka());
-  // forest output
-  CU_TRY(cudaMemsetAsync(ctx_->d_counters + kCMisc, 0, sizeof(DevCounters), st_));
-  if (msf_count_ > 0 && forest_bits_) {
+  // forest output (written by the cooperative rounds themselves)
+  if (!coop_done_) CU_TRY(cudaMemsetAsync(ctx_->d_counters + kCMisc, 0, sizeof(DevCounters), st_));
+  if (coop_done_) {
+  } else if (msf_count_ > 0 && forest_bits_) {
     const int tm = tick();
     // the weight stays 0 here: the caller's split sums it per graph
     k_mark_forest<<<grid_for(msf_count_), kBlock, 0, st_>>>(msf_count_, msf_, forest_bits_);
@@ -1268,9 +1506,14 @@ kamsta_status Solve::run(Algo algo, kamsta_wedge* d_out, SolveOut* out) {
     account(KAMSTA_PHASE_EMIT, (msf_count_ - k0) * (4 + 12 + 12), 1);
   }
   CU_TRY(cudaEventRecord(ctx_->ev1, st_));
-  KS_TRY(fetch_counters());
   out->count = msf_count_;
-  out->weight = ctx_->h_counters[kCMisc].weight;
+  if (coop_done_) {
+    out->weight = static_cast<const coop::State*>(ctx_->h_state)->weight;
+    if (stats_) CU_TRY(cudaEventSynchronize(ctx_->ev1));
+  } else {
+    KS_TRY(fetch_counters());
+    out->weight = ctx_->h_counters[kCMisc].weight;
+  }
   if (stats_) {
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx_->ev0, ctx_->ev1);

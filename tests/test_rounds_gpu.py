@@ -50,3 +50,81 @@ def test_class_plan_follows_the_sorted_sample(kamsta, oracle, n, m, wmax):
     assert np.array_equal(oracle.canon_keys(got), oracle.canon_keys(ref))
     assert st["levels"] == _planned_classes(e, n, 99)
     ctx.close()
+
+
+def _dev_solve(kamsta, ctx, edges, n, cfg, fn="boruvka_dev", shift=0):
+    """The forest as it lies in the output buffer, with its weight."""
+    import torch
+    flat = torch.zeros(3 * (len(edges) + shift), dtype=torch.int32, device="cuda")
+    flat[3 * shift:] = torch.from_numpy(edges.view(np.uint32).reshape(-1).view(np.int32)).cuda()
+    o = torch.zeros((n, 3), dtype=torch.int32, device="cuda")
+    st = {}
+    torch.cuda.synchronize()
+    k = getattr(ctx, fn)(flat.data_ptr() + 12 * shift, len(edges), n, o.data_ptr(), cfg, stats=st)
+    return o.cpu().numpy(), k, st
+
+
+def _rounds_case(oracle, name):
+    """Sizes around the cooperative rounds' limits: one CTA and many, a round
+    on either side of the vertices a CTA repeats on its own (4096), segment
+    counts, ragged tiles."""
+    kind, n, m, wmax = name
+    if kind == "gnm":
+        return oracle.gen_gnm(n, m, 7, wmax), n
+    if kind == "rgg":
+        return oracle.gen_rgg2d(n, oracle.rgg_radius(n, m), 9), n
+    if kind == "path":  # one hook chain through every vertex
+        return oracle.symmetric_from_undirected([(i, i + 1, i + 1) for i in range(n - 1)]), n
+    # star and a far, separate pair: a hub and finished components
+    und = [(0, i, 1 + i % 7) for i in range(1, n - 2)] + [(n - 2, n - 1, wmax)]
+    return oracle.symmetric_from_undirected(und), n
+
+
+@pytest.mark.parametrize("name", [
+    ("gnm", 2, 1, 254), ("gnm", 3, 3, 1), ("star", 5, 0, 9), ("gnm", 1023, 4093, 254),
+    ("gnm", 4096, 4097, 254), ("gnm", 4097, 50000, 1), ("gnm", 8193, 8190, 1 << 30),
+    ("path", 4099, 0, 0), ("path", 70001, 0, 0), ("star", 30011, 0, 254),
+    ("gnm", 30000, 1000003, 254), ("rgg", 20011, 12, 0), ("rgg", 400009, 9, 0),
+    ("gnm", 600011, 700001, 254)], ids=lambda c: f"{c[0]}-{c[1]}-{c[2]}")
+@pytest.mark.parametrize("lp", [0, 1])
+def test_cooperative_rounds_match_host_driven_rounds(kamsta, oracle, name, lp):
+    """The cooperative rounds write what the host-driven rounds write, byte
+    for byte (a traced solve runs the latter)."""
+    e, n = _rounds_case(oracle, name)
+    ctx = kamsta.Context(0)
+    got, k, st = _dev_solve(kamsta, ctx, e, n, kamsta.AlgorithmConfig(local_preprocessing=lp))
+    want, kw, sw = _dev_solve(kamsta, ctx, e, n,
+                              kamsta.AlgorithmConfig(local_preprocessing=lp, trace=True))
+    assert sw["trace_len"] == sw["rounds"] > 0
+    assert k == kw and st["total_weight"] == sw["total_weight"] and st["rounds"] == sw["rounds"]
+    assert np.array_equal(got, want)
+    if len(e) < 1 << 20:
+        ref, w = oracle.kruskal(e, n)
+        assert k == len(ref) and st["total_weight"] == w
+    # an input that starts off a 16-byte boundary
+    off, ko, _ = _dev_solve(kamsta, ctx, e, n, kamsta.AlgorithmConfig(local_preprocessing=lp),
+                            shift=1)
+    assert ko == kw and np.array_equal(off, want)
+    ctx.close()
+
+
+def test_cooperative_rounds_from_threads(kamsta, oracle):
+    """Solves on several threads and streams at once give what they give alone."""
+    import threading
+    graphs = [oracle.gen_gnm(20000 + 1000 * i, 150000, 50 + i) for i in range(4)]
+    cfg = kamsta.AlgorithmConfig(local_preprocessing=1)
+    ctxs = [kamsta.Context(0) for _ in graphs]
+    want = [_dev_solve(kamsta, c, e, 30000, cfg) for c, e in zip(ctxs, graphs)]
+    bad = []
+
+    def work(i):
+        for _ in range(10):
+            got, k, _ = _dev_solve(kamsta, ctxs[i], graphs[i], 30000, cfg)
+            if k != want[i][1] or not np.array_equal(got, want[i][0]):
+                bad.append(i)
+
+    th = [threading.Thread(target=work, args=(i,)) for i in range(len(graphs))]
+    [t.start() for t in th]
+    [t.join() for t in th]
+    assert not bad
+    [c.close() for c in ctxs]
