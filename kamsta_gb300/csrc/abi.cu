@@ -189,10 +189,11 @@ kamsta_status solve_7bit_locked(kamsta_ctx* ctx, const kamsta_cgraph& g, kamsta_
   cudaError_t e = ctx_alloc(ctx, &buf, g.m_directed * sizeof(kamsta_wedge), st);
   if (e != cudaSuccess) return cuda_status(e, "decode buffer");
   struct Free {
+    kamsta_ctx* c;
     void* p;
     cudaStream_t s;
-    ~Free() { cudaFreeAsync(p, s); }
-  } fr{buf, st};
+    ~Free() { ctx_free(c, p, s); }
+  } fr{ctx, buf, st};
   e = cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), st);
   if (e != cudaSuccess) return cuda_status(e, "cudaMemsetAsync");
   kamsta_status s = decode_7bit(g, static_cast<kamsta_wedge*>(buf), ctx->d_err, st);
@@ -300,10 +301,11 @@ kamsta_status solve_cgraph_host(Algo algo, const kamsta_cgraph* g, kamsta_cfg c,
   e = ctx_alloc(ctx, &buf, g->m_directed * sizeof(kamsta_wedge), st);
   if (e != cudaSuccess) return cuda_status(e, "decode buffer");
   struct Free {
+    kamsta_ctx* c;
     void* p;
     cudaStream_t s;
-    ~Free() { cudaFreeAsync(p, s); }
-  } fr{buf, st};
+    ~Free() { ctx_free(c, p, s); }
+  } fr{ctx, buf, st};
   kamsta_wedge* dec = static_cast<kamsta_wedge*>(buf);
   dg.chunk_offset = doff;
   dg.chunk_first = dfirst;
@@ -508,6 +510,7 @@ kamsta_status kamsta_ctx_destroy(kamsta_ctx* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->aux) cudaStreamSynchronize(ctx->aux);
   ctx->fixed.release();
+  heap_release(ctx);
   if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   if (ctx->d_counters) cudaFree(ctx->d_counters);
   if (ctx->d_err) cudaFree(ctx->d_err);
@@ -538,6 +541,8 @@ kamsta_status kamsta_ctx_trim(kamsta_ctx* ctx) {
   std::lock_guard<std::mutex> lock(ctx->mu);
   ctx->fixed.release();
   ctx->io.release();
+  heap_release(ctx);
+  ctx->heap.want = 0;
   if (ctx->pool) {
     cudaStreamSynchronize(ctx->stream);
     cudaMemPoolTrimTo(ctx->pool, 0);
@@ -552,6 +557,11 @@ kamsta_status kamsta_ctx_set_memory_limit(kamsta_ctx* ctx, uint64_t bytes) {
   }
   std::lock_guard<std::mutex> lock(ctx->mu);
   ctx->mem_limit = bytes;
+  ctx->heap.off = false;
+  if (bytes && ctx_device_bytes(ctx) > bytes) {  // what only serves speed goes first
+    heap_release(ctx);
+    ctx->heap.want = 0;
+  }
   return KAMSTA_OK;
 }
 
@@ -559,7 +569,7 @@ uint64_t kamsta_ctx_pool_bytes(const kamsta_ctx* ctx) {
   if (!ctx) return 0;
   uint64_t pool = 0;
   if (ctx->pool) cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &pool);
-  return ctx->fixed.cap + ctx->io.cap + pool;
+  return ctx->fixed.cap + ctx->io.cap + ctx->heap.cap + pool;
 }
 
 kamsta_status kamsta_mst_boruvka(const kamsta_wedge* edges, uint64_t m, uint32_t n,

@@ -335,14 +335,16 @@ inline size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 struct PoolBuf {
   void* p = nullptr;
   cudaStream_t st = nullptr;
+  kamsta_ctx* c = nullptr;
   ~PoolBuf() { reset(); }
   void reset() {
-    if (p) cudaFreeAsync(p, st);
+    if (p) ctx_free(c, p, st);
     p = nullptr;
   }
   cudaError_t alloc(kamsta_ctx* ctx, size_t bytes, cudaStream_t s) {
     reset();
     st = s;
+    c = ctx;
     return ctx_alloc(ctx, &p, std::max<size_t>(bytes, 256), s);
   }
 };
@@ -698,9 +700,9 @@ kamsta_status solve_union(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint
 
 bool is_small_graph(const kamsta_ctx* ctx, const kamsta_graph_desc& g) { return is_small(ctx, g); }
 
-kamsta_status solve_wave(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint32_t G,
-                         const kamsta_cfg& cfg, bool host_buffers, cudaStream_t st,
-                         BatchWaveStats* ws) {
+static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint32_t G,
+                                     const kamsta_cfg& cfg, bool host_buffers, cudaStream_t st,
+                                     BatchWaveStats* ws) {
   std::vector<uint32_t> sm, lg;
   for (uint32_t i = 0; i < G; ++i)
     ((!host_buffers && is_small(ctx, g[i])) ? sm : lg).push_back(i);
@@ -750,6 +752,20 @@ kamsta_status solve_wave(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint3
   ws->launches = us.launches + launches;
   ws->solve_ms = us.solve_ms;
   return KAMSTA_OK;
+}
+
+kamsta_status solve_wave(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint32_t G,
+                         const kamsta_cfg& cfg, bool host_buffers, cudaStream_t st,
+                         BatchWaveStats* ws) {
+  auto once = [&]() -> kamsta_status {
+    HeapScope scope(ctx, st);
+    const kamsta_status s = solve_wave_once(ctx, algo, g, G, cfg, host_buffers, st, ws);
+    if (s == KAMSTA_OK) scope.finished();
+    return s;
+  };
+  kamsta_status s = once();
+  if (s == KAMSTA_E_OOM && heap_retry(ctx)) s = once();
+  return s;
 }
 
 // Autotuner of the batch path: times the persistent small-graph kernel at

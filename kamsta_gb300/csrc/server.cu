@@ -75,7 +75,7 @@ uint64_t wave_peak_bytes(kamsta_ctx* ctx) {
     cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemHigh, &high);
     cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrUsedMemHigh, &zero);
   }
-  return high + ctx->fixed.cap + ctx->io.cap;
+  return high + ctx->fixed.cap + ctx->io.cap + ctx->heap.cap;
 }
 }  // namespace
 }  // namespace kamsta

@@ -58,17 +58,142 @@ cudaError_t Arena::reserve(size_t bytes) {
   return cudaSuccess;
 }
 
+void* Heap::take(size_t bytes) {
+  bytes = (bytes + 255) & ~static_cast<size_t>(255);
+  size_t best = free_list.size();
+  for (size_t i = 0; i < free_list.size(); ++i)
+    if (free_list[i].size >= bytes &&
+        (best == free_list.size() || free_list[i].size < free_list[best].size))
+      best = i;
+  if (best == free_list.size()) return nullptr;
+  const size_t off = free_list[best].off;
+  used.push_back({off, bytes});
+  free_list[best].off += bytes;
+  free_list[best].size -= bytes;
+  if (free_list[best].size == 0) free_list.erase(free_list.begin() + static_cast<long>(best));
+  return base + off;
+}
+
+bool Heap::give(void* p) {
+  char* c = static_cast<char*>(p);
+  if (c < base || c >= base + cap) return false;
+  const size_t off = static_cast<size_t>(c - base);
+  for (size_t i = 0; i < used.size(); ++i) {
+    if (used[i].off != off) continue;
+    Region r = used[i];
+    used[i] = used.back();
+    used.pop_back();
+    live -= std::min(live, r.size);
+    size_t k = 0;
+    while (k < free_list.size() && free_list[k].off < r.off) ++k;
+    if (k < free_list.size() && r.off + r.size == free_list[k].off) {  // merge with the next
+      r.size += free_list[k].size;
+      free_list.erase(free_list.begin() + static_cast<long>(k));
+    }
+    if (k > 0 && free_list[k - 1].off + free_list[k - 1].size == r.off)
+      free_list[k - 1].size += r.size;
+    else
+      free_list.insert(free_list.begin() + static_cast<long>(k), r);
+    break;
+  }
+  return true;
+}
+
+void heap_release(kamsta_ctx* ctx) {
+  Heap& h = ctx->heap;
+  if (h.base) cudaFree(h.base);
+  h.base = nullptr;
+  h.cap = 0;
+  h.free_list.clear();
+  h.used.clear();
+}
+
+// After a call that ran out of memory: gives the heap's block back and keeps
+// the context on its pool alone.  True when that can help (nothing of the
+// heap is in use and it held memory).
+bool heap_retry(kamsta_ctx* ctx) {
+  if (ctx->heap.depth > 0 || ctx->heap.cap == 0) return false;
+  heap_release(ctx);
+  ctx->heap.off = true;
+  ctx->heap.want = 0;
+  return true;
+}
+
+HeapScope::HeapScope(kamsta_ctx* ctx, cudaStream_t st) : ctx_(ctx), st_(st) {
+  Heap& h = ctx->heap;
+  if (h.depth > 0) {
+    synced_ = true;  // the outermost scope waits
+    return;
+  }
+  opened_ = true;
+  h.depth = 1;
+  h.st = st;
+  h.live = 0;
+  // nothing of the heap is in use now; grow by replacing it
+  if (!h.off && h.want > h.cap &&
+      (!ctx->mem_limit || ctx_device_bytes(ctx) - h.cap + h.want <= ctx->mem_limit)) {
+    heap_release(ctx);
+    if (ctx->pool) cudaMemPoolTrimTo(ctx->pool, 0);
+    void* p = nullptr;
+    if (cudaMalloc(&p, h.want) == cudaSuccess) {
+      h.base = static_cast<char*>(p);
+      h.cap = h.want;
+    } else {
+      cudaGetLastError();
+      h.want = 0;
+    }
+  }
+  h.used.clear();
+  h.pooled.clear();
+  h.free_list.clear();
+  if (h.cap) h.free_list.push_back({0, h.cap});
+}
+
+HeapScope::~HeapScope() {
+  // blocks are handed out anew by the next call, on whatever stream: this
+  // call's work must be over
+  if (!synced_) cudaStreamSynchronize(st_);
+  if (!opened_) return;
+  ctx_->heap.depth = 0;
+  ctx_->heap.st = nullptr;
+}
+
 uint64_t ctx_device_bytes(const kamsta_ctx* ctx) {
   uint64_t used = 0;
   if (ctx->pool) cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used);
-  return used + ctx->fixed.cap + ctx->io.cap;
+  return used + ctx->fixed.cap + ctx->io.cap + ctx->heap.cap;
 }
 
 cudaError_t ctx_alloc(kamsta_ctx* ctx, void** p, size_t bytes, cudaStream_t st) {
   *p = nullptr;
+  Heap& h = ctx->heap;
+  const bool open = h.depth > 0 && h.st == st;
+  if (open) {
+    const size_t need = (bytes + 255) & ~static_cast<size_t>(255);
+    h.live += need;
+    h.want = std::max(h.want, h.live);
+    if ((*p = h.take(bytes)) != nullptr) return cudaSuccess;
+    // enough in all, but in pieces: some room more next time
+    if (h.live <= h.cap) h.want = std::max(h.want, h.cap + h.cap / 8 + need / 2);
+  }
   if (ctx->mem_limit && ctx_device_bytes(ctx) + bytes > ctx->mem_limit)
     return cudaErrorMemoryAllocation;
-  return cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+  const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+  if (open && e == cudaSuccess) h.pooled.push_back({*p, (bytes + 255) & ~static_cast<size_t>(255)});
+  return e;
+}
+
+void ctx_free(kamsta_ctx* ctx, void* p, cudaStream_t st) {
+  Heap& h = ctx->heap;
+  if (!p || h.give(p)) return;
+  for (auto& b : h.pooled)
+    if (b.first == p) {
+      h.live -= std::min(h.live, b.second);
+      b = h.pooled.back();
+      h.pooled.pop_back();
+      break;
+    }
+  cudaFreeAsync(p, st);
 }
 
 cudaError_t ctx_reserve(kamsta_ctx* ctx, Arena& a, size_t bytes) {
@@ -146,7 +271,7 @@ class Solve {
       free_list(L);
       delete L;
     }
-    if (coop_mem_) cudaFreeAsync(coop_mem_, st_);
+    if (coop_mem_) ctx_free(ctx_, coop_mem_, st_);
   }
 
   kamsta_status run(Algo algo, kamsta_wedge* d_out, SolveOut* out);
@@ -373,7 +498,7 @@ kamsta_status Solve::alloc_list(SegList* L, uint32_t nseg, uint64_t cap) {
 }
 
 void Solve::free_list(SegList* L) {
-  if (L && L->mem) cudaFreeAsync(L->mem, st_);
+  if (L && L->mem) ctx_free(ctx_, L->mem, st_);
   if (L) {
     L->mem = nullptr;
     L->base = nullptr;
@@ -674,7 +799,7 @@ kamsta_status Solve::dedupe(SegList* L, uint32_t nr) {
   cudaError_t e = radix_sort_pairs_u32(st_, keys, keys2, vals, vals2, phys, bits, counts, status,
                                        &ctx_->d_counters[kCMisc].ticket, ctx_->d_err, &alt, sms_);
   if (e != cudaSuccess) {
-    cudaFreeAsync(mem, st_);
+    ctx_free(ctx_, mem, st_);
     return cuda_status(e, "radix sort (dedupe)");
   }
   if (alt) {
@@ -683,7 +808,7 @@ kamsta_status Solve::dedupe(SegList* L, uint32_t nr) {
   }
   k_dedupe_mark<<<grid_for(phys), kBlock, 0, st_>>>(keys, vals, phys, wbits, L->base,
                                                    &ctx_->d_counters[kCMisc].cnt[3]);
-  CU_TRY(cudaFreeAsync(mem, st_));
+  ctx_free(ctx_, mem, st_);
   tock(KAMSTA_PHASE_DEDUPE, t0);
   const uint32_t passes = static_cast<uint32_t>((bits + 7) / 8);
   // wmax read; keys: record read + key/value write; per digit pass: upsweep
@@ -983,12 +1108,11 @@ kamsta_status Solve::contract_rows(uint32_t wmin, uint32_t wmax, SegList* E, boo
   void* smem = nullptr;
   CU_TRY(ctx_alloc(ctx_, &smem, sizeof(uint32_t) * (2 * uint64_t(cap_s) + nfence + 1), st_));
   struct Free {
+    kamsta_ctx* c;
     void* p;
     cudaStream_t s;
-    ~Free() {
-      if (p) cudaFreeAsync(p, s);
-    }
-  } fs{smem, st_};
+    ~Free() { ctx_free(c, p, s); }
+  } fs{ctx_, smem, st_};
   uint32_t* S = static_cast<uint32_t*>(smem);
   uint32_t* row_lo = S + cap_s;
   uint32_t* fence = row_lo + cap_s;
@@ -1022,7 +1146,7 @@ kamsta_status Solve::contract_rows(uint32_t wmin, uint32_t wmax, SegList* E, boo
                  ib = round_up(k * 4, 256), cb = round_up(rs.counts * 4, 256),
                  sb = round_up(rs.status * 8, 256);
     CU_TRY(ctx_alloc(ctx_, &tmem, rb + 2 * kb + 2 * ib + cb + sb, st_));
-    Free ft{tmem, st_};
+    Free ft{ctx_, tmem, st_};
     char* m = static_cast<char*>(tmem);
     Rec* tmp = reinterpret_cast<Rec*>(m);
     uint64_t* keys = reinterpret_cast<uint64_t*>(m + rb);
@@ -1540,10 +1664,28 @@ kamsta_status solve_device(kamsta_ctx* ctx, Algo algo, const kamsta_wedge* d_in,
                            kamsta_wedge* d_out, SolveOut* out, kamsta_stats* st,
                            cudaStream_t stream, uint32_t* d_forest_bits, HostIo* io) {
   if (st) std::memset(st, 0, sizeof(*st));
-  Solve s(ctx, stream ? stream : ctx->stream, d_in, m_directed, n, cfg, st);
-  s.forest_bits_ = d_forest_bits;
-  s.io_ = io;
-  return s.run(algo, d_out, out);
+  const cudaStream_t str = stream ? stream : ctx->stream;
+  auto once = [&]() -> kamsta_status {
+    HeapScope scope(ctx, str);
+    Solve s(ctx, str, d_in, m_directed, n, cfg, st);
+    s.forest_bits_ = d_forest_bits;
+    s.io_ = io;
+    const kamsta_status r = s.run(algo, d_out, out);
+    // a solve that ran to its end has waited for its last kernel
+    if (r == KAMSTA_OK) scope.finished();
+    return r;
+  };
+  kamsta_status r = once();
+  if (r == KAMSTA_E_OOM && heap_retry(ctx)) {
+    // the heap holds memory that the limit (or the device) needs elsewhere
+    if (st) std::memset(st, 0, sizeof(*st));
+    if (d_forest_bits && cudaMemsetAsync(d_forest_bits, 0, ((m_directed + 31) / 32) * 4, str) !=
+                             cudaSuccess)
+      return r;
+    if (io) io->early = 0;
+    r = once();
+  }
+  return r;
 }
 
 }  // namespace kamsta

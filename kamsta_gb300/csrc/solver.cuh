@@ -2,9 +2,11 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdint>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/kamsta_gpu.h"
@@ -30,6 +32,33 @@ struct Arena {
     off += bytes;
     return p;
   }
+};
+
+// One block of device memory that a context keeps for its solves' scratch and
+// divides on the host (best fit, neighbours merged).  The stream-ordered pool
+// serves the same requests, but a solve's lists differ in size, and the pool
+// then remaps physical memory for nearly each of them: 130 to 430 us of host
+// time per list of a few hundred MB (G(n,m) 2^26/2^30: 23.0 -> 20.3 ms per solve
+// with the heap).
+// A call opens the heap for its stream (HeapScope): blocks taken and given
+// back inside are reused in that stream's order only.  The block grows
+// between calls to what the largest call so far had live at once.
+struct Heap {
+  struct Region {
+    size_t off, size;
+  };
+  char* base = nullptr;
+  size_t cap = 0;
+  size_t want = 0;                 // size to grow to before the next call
+  size_t live = 0;                 // bytes out, here and in the pool, this call
+  std::vector<Region> free_list;   // by offset
+  std::vector<Region> used;
+  std::vector<std::pair<void*, size_t>> pooled;  // this call's blocks from the pool
+  cudaStream_t st = nullptr;       // the open call's stream
+  int depth = 0;                   // > 0: open
+  bool off = false;                // a memory limit left no room for it
+  void* take(size_t bytes);
+  bool give(void* p);              // false: not from here
 };
 
 // Per-kernel counter block in device memory (zeroed before each round).
@@ -62,7 +91,8 @@ struct kamsta_ctx {
   uint32_t tune_dir_items = 0;      // entries per thread of the first pass
   uint32_t tune_seg_items = 0;      // records per thread of the list passes
   kamsta::Arena fixed;   // vertex arrays and look-back words
-  cudaMemPool_t pool = nullptr;  // edge lists (stream-ordered, cached between calls)
+  cudaMemPool_t pool = nullptr;  // scratch outside a call's heap (stream-ordered, cached)
+  kamsta::Heap heap;             // scratch of the solves
   kamsta::DevCounters* d_counters = nullptr;  // kCSlots blocks
   uint32_t* d_samples = nullptr;               // weight samples (kSampleCap)
   uint32_t* d_err = nullptr;
@@ -124,7 +154,26 @@ kamsta_status cuda_status(cudaError_t e, const char* what);
 // scratch from its pool and the growth of its arenas.  Going over the limit
 // fails like a device allocation (cudaErrorMemoryAllocation -> KAMSTA_E_OOM).
 uint64_t ctx_device_bytes(const kamsta_ctx* ctx);
+// Scratch for work on `st`: from the heap while it is open for that stream,
+// else from the pool.  ctx_free takes either back.
 cudaError_t ctx_alloc(kamsta_ctx* ctx, void** p, size_t bytes, cudaStream_t st);
+void ctx_free(kamsta_ctx* ctx, void* p, cudaStream_t st);
+// Opens the context's heap for work on one stream until the scope ends; the
+// outermost scope grows it first and, unless finished() said that the stream
+// has been waited for, waits for the stream last.
+class HeapScope {
+ public:
+  HeapScope(kamsta_ctx* ctx, cudaStream_t st);
+  ~HeapScope();
+  void finished() { synced_ = true; }
+
+ private:
+  kamsta_ctx* ctx_;
+  cudaStream_t st_;
+  bool opened_ = false, synced_ = false;
+};
+void heap_release(kamsta_ctx* ctx);
+bool heap_retry(kamsta_ctx* ctx);
 cudaError_t ctx_reserve(kamsta_ctx* ctx, Arena& a, size_t bytes);
 
 }  // namespace kamsta

@@ -128,3 +128,44 @@ def test_cooperative_rounds_from_threads(kamsta, oracle):
     [t.join() for t in th]
     assert not bad
     [c.close() for c in ctxs]
+
+
+def test_scratch_heap_limits_and_trim(kamsta, oracle):
+    """A context's scratch block grows to what its largest call needed, is
+    counted, gives way to a memory limit and is given back by trim; results
+    stay the same throughout."""
+    n = 1 << 20
+    big, small = oracle.gen_gnm(n, 1 << 23, 3), oracle.gen_gnm(5000, 40000, 4)
+    cfg = kamsta.AlgorithmConfig(local_preprocessing=1)
+    ctx = kamsta.Context(0)
+    first, k0, _ = _dev_solve(kamsta, ctx, big, n, cfg)
+    for _ in range(3):
+        again, k, _ = _dev_solve(kamsta, ctx, big, n, cfg)
+        assert k == k0 and np.array_equal(again, first)
+        held = ctx.pool_bytes()
+    want, ks, _ = _dev_solve(kamsta, kamsta.Context(0), small, 5000, cfg)
+    got, k, _ = _dev_solve(kamsta, ctx, small, 5000, cfg)
+    assert k == ks and np.array_equal(got, want)
+    # tightest limit (a binary search) under which a fresh context solves it
+    lo, hi = 1 << 20, 4 << 30
+    while hi - lo > 8 << 20:
+        mid = (lo + hi) // 2
+        c = kamsta.Context(0)
+        c.set_memory_limit(mid)
+        try:
+            _dev_solve(kamsta, c, big, n, cfg)
+            hi = mid
+        except kamsta.KamstaError as e:
+            assert e.status == kamsta._native.E_OOM
+            lo = mid
+        c.close()
+    ctx.set_memory_limit(hi)  # still enough, whatever the context held before
+    for _ in range(3):
+        again, k, _ = _dev_solve(kamsta, ctx, big, n, cfg)
+        assert k == k0 and np.array_equal(again, first)
+    ctx.set_memory_limit(0)
+    ctx.trim()
+    assert ctx.pool_bytes() < held
+    again, k, _ = _dev_solve(kamsta, ctx, big, n, cfg)
+    assert k == k0 and np.array_equal(again, first)
+    ctx.close()
