@@ -62,6 +62,9 @@ struct State {
   uint32_t nreps;                   // dense labels in use
   uint32_t rounds, levels;
   uint32_t vsel;  // representatives are in Vn (1) or V (0)
+  // the last launch's rounds: vertices before each, and left after the last
+  uint32_t last_rounds;
+  uint32_t size[kMaxRounds + 1];
   // error bits per launch: a launch that follows an error does nothing, and
   // all of its CTAs must see the same, so no launch looks at its own word
   uint32_t errs[kMaxLaunch];
@@ -86,7 +89,13 @@ struct Args {
   uint32_t* cnt[2];
   uint32_t cap;
   uint32_t n;
-  uint32_t first;   // first launch of the solve: n labels, no state yet
+  uint32_t first;   // no state yet: nr0 labels, msf0 forest edges, V as given
+  uint32_t nr0;
+  // earlier rounds of the same contraction (host-driven): map and
+  // representative words they used, and their last representatives (or null)
+  uint32_t roff0, ooff0;
+  const uint32_t* orig0;
+  uint64_t msf0;
   uint32_t direct;  // round 0: minima keyed by partner, edges to out
   uint32_t finalize;
   Emit emit;
@@ -94,6 +103,7 @@ struct Args {
   uint64_t *minA, *minB, *tiny;  // tiny: 3 * kTinyN words
   uint32_t* vcnt;                // 2 per CTA
   uint32_t *out, *bits;
+  unsigned long long* weight;    // of the edges written to out
   uint32_t launch;
   State* st;
   const uint32_t* pass_err;  // error word of the passes before
@@ -467,7 +477,7 @@ __device__ void write_phase(Shared& s, const Args& a, uint32_t n, const uint64_t
   }
   if (direct) {
     wsum = warp_sum(wsum);
-    if (lane_id() == 0 && wsum) atomicAdd(&a.st->weight, static_cast<unsigned long long>(wsum));
+    if (lane_id() == 0 && wsum) atomicAdd(a.weight, static_cast<unsigned long long>(wsum));
   }
 }
 
@@ -638,13 +648,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_rounds(const __grid_constant__ 
     return;
   const uint32_t tid = threadIdx.x, gtid = blockIdx.x * kThreads + tid;
   const uint32_t gsz = gridDim.x * kThreads;
-  uint32_t nr = a.first ? a.n : st->nreps;
+  uint32_t nr = a.first ? a.nr0 : st->nreps;
   const uint32_t n0 = nr;
   const uint32_t vsel = a.first ? 0u : st->vsel;
   const uint32_t* V = vsel ? a.Vn : a.V;
   uint32_t* Vnext = vsel ? a.V : a.Vn;
-  const uint64_t msf_start = a.first ? 0ull : st->msf_count;
-  uint64_t msf_count = msf_start;
+  uint64_t msf_count = a.first ? a.msf0 : st->msf_count;
   unsigned long long sum_m = 0, sum_n = 0;
   for (uint32_t x = gtid; x < 3 * kTinyN; x += gsz) a.tiny[x] = kInf64;
   List cur{a.src, a.src_nseg, a.src_cap};
@@ -667,8 +676,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_rounds(const __grid_constant__ 
   }
   uint64_t* minv = a.minA;
   uint32_t tiny = 0;  // next of the three rotating arrays to receive minima
-  uint32_t r = 0, roff = 0, ooff = 0;
-  const uint32_t* orig_cur = V;
+  uint32_t r = 0, roff = a.roff0, ooff = a.ooff0;
+  const uint32_t* orig_cur = a.orig0 ? a.orig0 : V;
   uint32_t m = 0;
   if (nr > 1) m = seg_prefix32(s, cur_cnt, cur.nseg);
   while (m > 0) {
@@ -901,7 +910,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_rounds(const __grid_constant__ 
       }
     }
     local = warp_sum(local);
-    if (lane_id() == 0 && local) atomicAdd(&st->weight, static_cast<unsigned long long>(local));
+    if (lane_id() == 0 && local) atomicAdd(a.weight, static_cast<unsigned long long>(local));
   }
   // (a launch that is not the solve's first has passed a barrier after its
   // prologue, and with it every CTA's reads of the state)
@@ -912,6 +921,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_rounds(const __grid_constant__ 
     st->levels += 1;
     st->sum_m += sum_m;
     st->sum_n += sum_n;
+    st->last_rounds = r;
+    for (uint32_t k = 0; k < r; ++k) st->size[k] = s_size[k];
+    st->size[r] = nr;
     if (r > 0 && a.finalize) st->vsel = vsel ^ 1u;
   }
 }

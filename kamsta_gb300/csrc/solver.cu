@@ -241,6 +241,17 @@ constexpr uint32_t kWideRoundN = 1u << 16;
 // shared memory (32 KB).
 constexpr uint32_t kSminMax = 4096;
 
+// Larger inputs hand a contraction over once its list has at most kTailM
+// records (and 2^23 vertices): from there on a host-driven round's 60 us of
+// launches and reads outweigh its wider grid (us, host-driven / handed over:
+// filter-Boruvka 2^20/2^24 2390 / 1464, 7-bit 2^20/2^24 1890 / 1233, R-MAT
+// 2^22 1700 / 1435, RGG-2D 2^24 4800 / 4250).
+constexpr uint64_t kTailM = 1ull << 24;
+constexpr uint32_t kTailN = 1u << 23;
+// Largest n whose label update the cooperative grid does itself; beyond it
+// the update's gathers need the full occupancy of its own kernels.
+constexpr uint32_t kCoopFinalizeN = 1u << 22;
+
 template <typename K>
 static int blocks_per_sm(K kernel, size_t dyn_smem) {
   int per_sm = 1;
@@ -338,13 +349,33 @@ class Solve {
   // false when the solve has to run by host-driven rounds instead.
   bool coop_fits() const;
   kamsta_status run_coop(bool* done);
-  kamsta_status coop_launch(const SegList* L, uint64_t md, uint32_t wmin, uint32_t wmax,
-                            bool prologue, bool finalize, bool emit);
+  coop::Args coop_args(const SegList* L) const;
+  kamsta_status coop_launch(coop::Args a);
+  kamsta_status coop_buffers(uint64_t cap, SegList* reuse);
+  bool coop_options() const;  // the solve's options allow cooperative rounds
+  // All rounds left of a contraction whose list has become small enough, and
+  // (whole contractions over few vertices) the label update; false in *ran
+  // when there is no memory for the buffers.
+  struct Rounds {  // the rounds of one contraction so far
+    uint32_t nr = 0, r = 0;
+    uint64_t *minv = nullptr, *minn = nullptr;
+    size_t roff = 0, ooff = 0;
+    const uint32_t* orig_cur = nullptr;
+    uint32_t* maps[kMaxRounds];
+    const uint32_t* origs[kMaxRounds + 1];
+    uint32_t sizes[kMaxRounds];
+  };
+  kamsta_status coop_tail(SegList* L, bool own, bool prologue, Rounds* R, bool* ran,
+                          bool* finalized);
+  kamsta_status early_forest(uint64_t added);
+  kamsta_status finish_rounds(const Rounds& R, uint32_t n0);
   kamsta_status coop_reset();
   kamsta_status coop_fetch();
   uint32_t coop_grid_ = 0, coop_launches_ = 0;
+  bool coop_off_ = false;     // the buffers did not fit once
   uint64_t coop_cap_ = 0;     // records per segment of the two buffers
   Rec* coop_buf_[2] = {nullptr, nullptr};
+  SegList* coop_list_[2] = {nullptr, nullptr};  // what holds them
   bool coop_done_ = false;    // the solve's forest is written
   kamsta_status run_filter_boruvka();
   // ---- debugging (KAMSTA_DEBUG_CHECKS=1): host-side invariant checks
@@ -819,28 +850,48 @@ kamsta_status Solve::dedupe(SegList* L, uint32_t nr) {
   return KAMSTA_OK;
 }
 
+// The first round's forest edges, written directly: send them to the host
+// (host entry points) while the solve goes on.
+kamsta_status Solve::early_forest(uint64_t added) {
+  if (!io_ || !io_->host_out || added == 0) return KAMSTA_OK;
+  CU_TRY(cudaEventRecord(io_->ev_early, st_));
+  CU_TRY(cudaStreamWaitEvent(io_->copy_stream, io_->ev_early, 0));
+  CU_TRY(cudaMemcpyAsync(io_->host_out, d_out_, added * sizeof(kamsta_wedge),
+                         cudaMemcpyDeviceToHost, io_->copy_stream));
+  io_->early = added;
+  return KAMSTA_OK;
+}
+
 kamsta_status Solve::rounds(SegList* L, bool own) {
   levels_++;
   const uint32_t n0 = nreps_;
   SegList* cur = L;
   bool cur_owned = own;
-  uint32_t nr = n0;
-  uint64_t* minv = minA_;
-  uint64_t* minn = minB_;
   // per round: its map, its vertices' original representatives, its size
-  uint32_t* maps[kMaxRounds];
-  const uint32_t* origs[kMaxRounds + 1];
-  uint32_t sizes[kMaxRounds];
-  origs[0] = V_;
-  size_t roff = 0, ooff = 0;
-  uint32_t r = 0;
-  const uint32_t* orig_cur = V_;
+  Rounds rs;
+  rs.nr = n0;
+  rs.minv = minA_;
+  rs.minn = minB_;
+  rs.origs[0] = rs.orig_cur = V_;
+  uint32_t& nr = rs.nr;
+  uint32_t& r = rs.r;
+  bool finalized = false;
   while (cur->total > 0) {
+    if (coop_options() && cur->total <= kTailM && nr <= kTailN) {
+      bool ran = false;
+      KS_TRY(coop_tail(cur, cur_owned, false, &rs, &ran, &finalized));
+      if (ran) break;
+    }
     if (r >= static_cast<uint32_t>(kMaxRounds)) {
       set_error("round cap reached");
       return KAMSTA_E_NOCONVERGE;
     }
     trace(cur->total, nr);
+    uint64_t*& minv = rs.minv;
+    uint64_t*& minn = rs.minn;
+    size_t& roff = rs.roff;
+    size_t& ooff = rs.ooff;
+    const uint32_t*& orig_cur = rs.orig_cur;
     const uint64_t m = cur->total;
     if (!(cfg_.flags & KAMSTA_FLAG_DEDUPE_NEVER) &&
         ((cfg_.flags & KAMSTA_FLAG_DEDUPE_ALWAYS) ||
@@ -916,14 +967,7 @@ kamsta_status Solve::rounds(SegList* L, bool own) {
             tagged ? 4 : 5);
     if (direct) {
       direct_count_ = added;
-      if (io_ && io_->host_out && added > 0) {
-        // final already: send them to the host while the solve goes on
-        CU_TRY(cudaEventRecord(io_->ev_early, st_));
-        CU_TRY(cudaStreamWaitEvent(io_->copy_stream, io_->ev_early, 0));
-        CU_TRY(cudaMemcpyAsync(io_->host_out, d_out_, added * sizeof(kamsta_wedge),
-                               cudaMemcpyDeviceToHost, io_->copy_stream));
-        io_->early = added;
-      }
+      KS_TRY(early_forest(added));  // final already
     }
     if (debug_) {
       fprintf(stderr, "[kamsta debug] round %u: m=%llu n=%u -> m'=%llu n'=%llu forest+=%llu\n", r,
@@ -937,9 +981,9 @@ kamsta_status Solve::rounds(SegList* L, bool own) {
       set_error("internal: forest larger than n-1");
       return KAMSTA_E_CUDA;
     }
-    maps[r] = R;
-    sizes[r] = nr;
-    origs[r + 1] = onext;
+    rs.maps[r] = R;
+    rs.sizes[r] = nr;
+    rs.origs[r + 1] = onext;
     roff += nr;
     ooff += n_next;
     orig_cur = onext;
@@ -953,7 +997,16 @@ kamsta_status Solve::rounds(SegList* L, bool own) {
   if (cur_owned) free_list(cur);
   rounds_ += r;
   if (r == 0) return KAMSTA_OK;  // nothing contracted; labels unchanged
-  if (final_contraction_) return KAMSTA_OK;  // no later pass needs the labels
+  if (final_contraction_ || finalized) return KAMSTA_OK;  // no later pass needs the labels
+  return finish_rounds(rs, n0);
+}
+
+// The labels after a contraction: composed over its rounds' maps.
+kamsta_status Solve::finish_rounds(const Rounds& rs, uint32_t n0) {
+  const uint32_t r = rs.r;
+  uint32_t* const* maps = rs.maps;
+  const uint32_t* const* origs = rs.origs;
+  const uint32_t* sizes = rs.sizes;
   const int tf = tick();
   CU_TRY(cudaMemsetAsync(ctx_->d_counters + kCRep, 0, sizeof(DevCounters), st_));
   RepScanArgs ra{};
@@ -1186,6 +1239,24 @@ kamsta_status Solve::contract_rows(uint32_t wmin, uint32_t wmax, SegList* E, boo
 kamsta_status Solve::contract(const SegList* L, uint32_t wmin, uint32_t wmax, double frac) {
   if ((L && L->total == 0) || nreps_ <= 1) return KAMSTA_OK;
   fill_inf(minA_, nreps_);
+  if (L && coop_options() && L->total <= kTailM && n_ <= kTailN) {
+    // relabelled, contracted and finished by one cooperative launch; its
+    // labels lie in the L2, so no membership bitmap is needed
+    Rounds rs;
+    rs.nr = nreps_;
+    rs.minv = minA_;
+    rs.minn = minB_;
+    rs.origs[0] = rs.orig_cur = V_;
+    const uint32_t n0 = nreps_;
+    bool ran = false, finalized = false;
+    KS_TRY(coop_tail(const_cast<SegList*>(L), false, true, &rs, &ran, &finalized));
+    if (ran) {
+      levels_++;
+      rounds_ += rs.r;
+      if (rs.r == 0 || final_contraction_ || finalized) return KAMSTA_OK;
+      return finish_rounds(rs, n0);
+    }
+  }
   KS_TRY(pick_big(&big_label_, &use_big_));
   if (!L && use_big_) {  // heaviest class of the directed input: row scans
     SegList* E = new_list();
@@ -1243,13 +1314,44 @@ cudaError_t launch_in_order(int dev, const void* f, uint32_t grid, uint32_t bloc
 // by row scans than by the stream used here (2^26: 400 MB of reads).
 constexpr uint64_t kCoopMaxMd = (1ull << 25) - 1;
 
-bool Solve::coop_fits() const {
+bool Solve::coop_options() const {
   // per-round traces, dedupe between rounds and the debug checks are the
   // host-driven rounds' alone
-  if (debug_ || (cfg_.flags & (KAMSTA_FLAG_TRACE | KAMSTA_FLAG_DEDUPE_ALWAYS))) return false;
+  if (debug_ || coop_off_ || (cfg_.flags & (KAMSTA_FLAG_TRACE | KAMSTA_FLAG_DEDUPE_ALWAYS)))
+    return false;
   if (cfg_.dedupe_ratio && !(cfg_.flags & KAMSTA_FLAG_DEDUPE_NEVER)) return false;
-  return n_ >= 2 && n_ < kRootTag && md_ <= kCoopMaxMd &&
-         bounds_.size() + 1 <= coop::kMaxLaunch;
+  return n_ >= 2 && n_ < kRootTag;
+}
+
+bool Solve::coop_fits() const {
+  return coop_options() && md_ <= kCoopMaxMd && bounds_.size() + 1 <= coop::kMaxLaunch;
+}
+
+// One CTA per SM; little work takes fewer, so that its barriers are short.
+static uint32_t coop_grid(uint64_t work, int sms) {
+  const uint64_t step = uint64_t(coop::kThreads) * coop::kItems;
+  return static_cast<uint32_t>(std::max<uint64_t>(
+      1, std::min<uint64_t>(std::min(sms, kMaxSeg / coop::kGroups), (work + step - 1) / step)));
+}
+
+// Two list buffers of cap records per segment; `reuse` (a list read for the
+// last time before the second buffer is written) serves as the second when it
+// is large enough.
+kamsta_status Solve::coop_buffers(uint64_t cap, SegList* reuse) {
+  const uint32_t nq = coop_grid_ * coop::kGroups;
+  coop_cap_ = std::max<uint64_t>(cap, 1);
+  for (SegList*& B : coop_list_)
+    if (!B) B = new_list();
+  KS_TRY(alloc_list(coop_list_[0], nq, coop_cap_));
+  coop_buf_[0] = coop_list_[0]->base;
+  if (reuse && reuse->nseg * reuse->cap >= nq * coop_cap_) {
+    coop_buf_[1] = reuse->base;
+    return KAMSTA_OK;
+  }
+  const kamsta_status s = alloc_list(coop_list_[1], nq, coop_cap_);
+  coop_buf_[1] = coop_list_[1]->base;
+  if (s != KAMSTA_OK) free_list(coop_list_[0]);
+  return s;
 }
 
 // The state, the tiny rounds' minima and the buffers' counts come from the
@@ -1270,8 +1372,7 @@ kamsta_status Solve::coop_reset() {
   return KAMSTA_OK;
 }
 
-kamsta_status Solve::coop_launch(const SegList* L, uint64_t md, uint32_t wmin, uint32_t wmax,
-                                 bool prologue, bool finalize, bool emit) {
+coop::Args Solve::coop_args(const SegList* L) const {
   coop::Args a{};
   if (L) {
     a.src = L->base;
@@ -1280,20 +1381,14 @@ kamsta_status Solve::coop_launch(const SegList* L, uint64_t md, uint32_t wmin, u
     a.src_nseg = L->nseg;
   }
   a.in = in_;
-  a.md = static_cast<uint32_t>(md);
-  a.wmin = wmin;
-  a.wmax = wmax;
-  a.prologue = prologue ? 1u : 0u;
+  a.md = static_cast<uint32_t>(md_);
+  a.wmax = 0xffffffffu;
   for (int k = 0; k < 2; ++k) {
     a.buf[k] = coop_buf_[k];
     a.cnt[k] = coop_cnt_ + k * kMaxSeg;
   }
   a.cap = static_cast<uint32_t>(coop_cap_);
-  a.n = n_;
-  a.first = coop_launches_ == 0 ? 1u : 0u;
-  a.direct = direct_emit_ && coop_launches_ == 0 ? 1u : 0u;
-  a.finalize = finalize ? 1u : 0u;
-  a.emit = !emit ? coop::Emit::kNone : forest_bits_ ? coop::Emit::kBits : coop::Emit::kEdges;
+  a.n = a.nr0 = n_;
   a.P = P_;
   a.D = D_;
   a.V = V_;
@@ -1310,10 +1405,15 @@ kamsta_status Solve::coop_launch(const SegList* L, uint64_t md, uint32_t wmin, u
   a.vcnt = cta_counts_;
   a.out = reinterpret_cast<uint32_t*>(d_out_);
   a.bits = forest_bits_;
-  a.launch = coop_launches_;
+  a.weight = &coop_state_->weight;
   a.st = coop_state_;
   a.pass_err = ctx_->d_err;
+  a.launch = coop_launches_;
   a.err = &coop_state_->errs[coop_launches_];
+  return a;
+}
+
+kamsta_status Solve::coop_launch(coop::Args a) {
   void* args[] = {&a};
   const int t0 = tick();
   CU_TRY(launch_in_order(ctx_->device, reinterpret_cast<const void*>(&coop::k_rounds), coop_grid_,
@@ -1336,12 +1436,7 @@ kamsta_status Solve::run_coop(bool* done) {
   const int K = static_cast<int>(b.size());
   const int nmat = std::max(1, std::min(K, kMaxOut));
   SegList* C[kMaxOut] = {new_list(), new_list(), new_list()};
-  // one CTA per SM; small graphs take fewer, so that their barriers are short
-  const uint64_t work = md_ / 2 + n_;
-  const uint64_t step = uint64_t(coop::kThreads) * coop::kItems;
-  coop_grid_ = static_cast<uint32_t>(
-      std::max<uint64_t>(1, std::min<uint64_t>(std::min(sms_, kMaxSeg / coop::kGroups),
-                                               (work + step - 1) / step)));
+  coop_grid_ = coop_grid(md_ / 2 + n_, sms_);
   const kamsta_status s = [&]() -> kamsta_status {
     KS_TRY(first_pass(C, nmat, false));
     // a list holds at most one copy of each edge; the classes left in the
@@ -1354,26 +1449,25 @@ kamsta_status Solve::run_coop(bool* done) {
       const double f = std::min(1.0, sample_share(samples_host_, b[c - 1] + 1,
                                                   c < K ? b[c] : 0xffffffffu));
       const uint64_t chunk = (md_ + nq - 1) / nq;
-      const double est = f * chunk * 1.1 + 6.0 * std::sqrt(f * chunk) + step;
+      const double est =
+          f * chunk * 1.1 + 6.0 * std::sqrt(f * chunk) + coop::kThreads * coop::kItems;
       cap = std::max(cap, std::min<uint64_t>(chunk, static_cast<uint64_t>(est)));
     }
-    coop_cap_ = cap;
-    SegList* B0 = new_list();
-    KS_TRY(alloc_list(B0, nq, cap));
-    coop_buf_[0] = B0->base;
-    if (K == 0 && C[0]->nseg * C[0]->cap >= nq * cap) {
-      coop_buf_[1] = C[0]->base;  // read for the last time before it is written
-    } else {
-      SegList* B1 = new_list();
-      KS_TRY(alloc_list(B1, nq, cap));
-      coop_buf_[1] = B1->base;
-    }
+    KS_TRY(coop_buffers(cap, K == 0 ? C[0] : nullptr));
     KS_TRY(coop_reset());
     for (int c = 0; c <= std::max(K, nmat - 1); ++c) {
       const bool last = c == std::max(K, nmat - 1);
       const uint32_t lo = c < nmat ? 0u : b[c - 1] + 1;
       const uint32_t hi = c < nmat || c >= K ? 0xffffffffu : b[c];
-      KS_TRY(coop_launch(c < nmat ? C[c] : nullptr, md_, lo, hi, c > 0, !last, last));
+      coop::Args a = coop_args(c < nmat ? C[c] : nullptr);
+      a.wmin = lo;
+      a.wmax = hi;
+      a.first = c == 0 ? 1u : 0u;
+      a.direct = direct_emit_ && c == 0 ? 1u : 0u;
+      a.prologue = c > 0 ? 1u : 0u;
+      a.finalize = last ? 0u : 1u;
+      if (last) a.emit = forest_bits_ ? coop::Emit::kBits : coop::Emit::kEdges;
+      KS_TRY(coop_launch(a));
     }
     return coop_fetch();
   }();
@@ -1389,6 +1483,7 @@ kamsta_status Solve::run_coop(bool* done) {
   if (s == KAMSTA_E_INPUT) return s;
   if (s != KAMSTA_OK || err != 0) {
     cudaGetLastError();
+    coop_off_ = true;
     k_init_vertices<<<grid_for(n_), kBlock, 0, st_>>>(n_, minA_, P_, V_, D_);
     CU_TRY(cudaMemsetAsync(dweight_, 0, sizeof(unsigned long long), st_));
     CU_TRY(cudaMemsetAsync(ctx_->d_err, 0, sizeof(uint32_t), st_));
@@ -1404,6 +1499,68 @@ kamsta_status Solve::run_coop(bool* done) {
   account(KAMSTA_PHASE_ROUND_EDGES, h.sum_m * 56 + h.sum_n * 60, coop_launches_);
   coop_done_ = true;
   *done = true;
+  return KAMSTA_OK;
+}
+
+kamsta_status Solve::coop_tail(SegList* L, bool own, bool prologue, Rounds* R, bool* ran,
+                               bool* finalized) {
+  *ran = false;
+  coop_grid_ = coop_grid(L->total + R->nr, sms_);
+  const uint32_t nq = coop_grid_ * coop::kGroups;
+  const kamsta_status s = [&]() -> kamsta_status {
+    KS_TRY(coop_buffers((L->total + nq - 1) / nq, own ? L : nullptr));
+    return coop_reset();
+  }();
+  if (s == KAMSTA_E_OOM) {
+    coop_off_ = true;
+    return KAMSTA_OK;
+  }
+  KS_TRY(s);
+  *ran = true;
+  const bool direct = direct_emit_ && R->r == 0;
+  *finalized = R->r == 0 && !final_contraction_ && n_ <= kCoopFinalizeN;
+  coop::Args a = coop_args(L);
+  a.first = 1;
+  a.nr0 = R->nr;
+  a.msf0 = msf_count_;
+  a.roff0 = static_cast<uint32_t>(R->roff);
+  a.ooff0 = static_cast<uint32_t>(R->ooff);
+  a.orig0 = R->orig_cur;
+  a.minA = R->minv;
+  a.minB = R->minn;
+  a.direct = direct ? 1u : 0u;
+  a.weight = dweight_;
+  a.prologue = prologue ? 1u : 0u;
+  a.finalize = *finalized ? 1u : 0u;
+  KS_TRY(coop_launch(a));
+  const kamsta_status fs = coop_fetch();
+  for (SegList* B : coop_list_) free_list(B);
+  KS_TRY(fs);
+  const coop::State& h = *static_cast<const coop::State*>(ctx_->h_state);
+  if (h.errs[0] != 0) {
+    *ctx_->h_err = h.errs[0];
+    return check_err();
+  }
+  for (uint32_t k = 0; k < h.last_rounds; ++k) {
+    R->maps[R->r] = Rbuf_ + R->roff;
+    R->sizes[R->r] = h.size[k];
+    R->origs[R->r + 1] = Obuf_ + R->ooff;
+    R->roff += h.size[k];
+    R->ooff += h.size[k + 1];
+    ++R->r;
+  }
+  R->nr = h.size[h.last_rounds];
+  const uint64_t added = h.msf_count - msf_count_;
+  msf_count_ = h.msf_count;
+  if (direct && h.last_rounds > 0) {
+    direct_count_ = h.direct_count;
+    KS_TRY(early_forest(direct_count_));
+  }
+  account(KAMSTA_PHASE_ROUND_EDGES, h.sum_m * 56 + h.sum_n * 60 + added * 8, 1);
+  if (*finalized && h.last_rounds > 0) {
+    nreps_ = h.nreps;
+    std::swap(V_, Vn_);
+  }
   return KAMSTA_OK;
 }
 
