@@ -465,10 +465,10 @@ kamsta_status kamsta_ctx_create(int device, kamsta_ctx** out) {
       (e = cudaEventCreateWithFlags(&c->ev_early, cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaMalloc(&c->d_counters, sizeof(DevCounters) * kCSlots)) != cudaSuccess ||
       (e = cudaMalloc(&c->d_err, sizeof(uint32_t))) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_samples, sizeof(uint32_t) * kSampleCap)) != cudaSuccess ||
+      (e = cudaMalloc(&c->d_samples, sizeof(uint32_t) * kSampleWords)) != cudaSuccess ||
       (e = cudaMallocHost(&c->h_counters, sizeof(DevCounters) * kCSlots)) != cudaSuccess ||
       (e = cudaMallocHost(&c->h_err, sizeof(uint32_t))) != cudaSuccess ||
-      (e = cudaMallocHost(&c->h_samples, sizeof(uint32_t) * kSampleCap)) != cudaSuccess ||
+      (e = cudaMallocHost(&c->h_samples, sizeof(uint32_t) * kSampleWords)) != cudaSuccess ||
       (e = cudaMallocHost(&c->h_state, kHostState)) != cudaSuccess ||
       (e = cudaEventCreate(&c->ev0)) != cudaSuccess ||
       (e = cudaEventCreate(&c->ev1)) != cudaSuccess) {

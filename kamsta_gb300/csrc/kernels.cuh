@@ -1682,14 +1682,112 @@ __global__ void k_mark_forest(uint64_t k, const uint32_t* __restrict__ msf,
   }
 }
 
+// The forest bitmap as a list of records in input order with original ids,
+// and the round-0 minima of its edges keyed by partner (both endpoints: a
+// record is all there is of its edge).  CTA c owns words [c * chunk, ...);
+// k_bits_count counts its bits, k_bits_list places its records behind those
+// of the CTAs before it.
+__global__ void __launch_bounds__(kBlock)
+    k_bits_count(const uint32_t* __restrict__ bits, uint64_t words, uint64_t chunk,
+                 uint32_t* __restrict__ cta_counts) {
+  const uint64_t lo = blockIdx.x * chunk, hi = lo + chunk < words ? lo + chunk : words;
+  uint32_t c = 0;
+  for (uint64_t q = lo + threadIdx.x; q < hi; q += kBlock) c += __popc(bits[q]);
+  __shared__ uint32_t s_c;
+  if (threadIdx.x == 0) s_c = 0;
+  __syncthreads();
+  c = warp_sum(c);
+  if (lane_id() == 0 && c) atomicAdd(&s_c, c);
+  __syncthreads();
+  if (threadIdx.x == 0) cta_counts[blockIdx.x] = s_c;
+}
+
+__global__ void __launch_bounds__(kBlock)
+    k_bits_list(const uint32_t* __restrict__ bits, uint64_t words, uint64_t chunk,
+                const uint32_t* __restrict__ cta_counts, const uint32_t* __restrict__ in,
+                uint64_t cap, Rec* __restrict__ out, uint64_t* minval, uint32_t* count) {
+  constexpr int kWarps = kBlock / 32;
+  __shared__ uint32_t s_w[2][kWarps];
+  __shared__ uint32_t s_base;
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  if (threadIdx.x < 32) {
+    uint32_t b = 0, t = 0;
+    for (uint32_t c = threadIdx.x; c < gridDim.x; c += 32) {
+      t += cta_counts[c];
+      if (c < blockIdx.x) b += cta_counts[c];
+    }
+    b = warp_sum(b);
+    t = warp_sum(t);
+    if (threadIdx.x == 0) {
+      s_base = b;
+      if (blockIdx.x == 0) *count = t;
+    }
+  }
+  __syncthreads();
+  uint64_t run = s_base;
+  const uint64_t lo = blockIdx.x * chunk, hi = lo + chunk < words ? lo + chunk : words;
+  int flip = 0;
+  for (uint64_t q0 = lo; q0 < hi; q0 += kBlock, flip ^= 1) {
+    const uint64_t q = q0 + threadIdx.x;
+    uint32_t f = q < hi ? bits[q] : 0u;
+    const uint32_t c = __popc(f);
+    uint32_t incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, incl, o);
+      if (lane >= static_cast<uint32_t>(o)) incl += y;
+    }
+    if (lane == 31) s_w[flip][warp] = incl;
+    __syncthreads();
+    uint32_t pre = 0, tot = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const uint32_t x = s_w[flip][w];
+      if (static_cast<uint32_t>(w) < warp) pre += x;
+      tot += x;
+    }
+    uint64_t k = run + pre + incl - c;
+    while (f) {
+      const uint32_t pos = static_cast<uint32_t>(q * 32 + (__ffs(f) - 1));
+      f &= f - 1;
+      const uint32_t* e = in + 3ull * pos;
+      const Rec r{e[0], e[1], e[2], pos};
+      if (k < cap) {
+        st_stream(out + k, r);
+        const uint64_t w = static_cast<uint64_t>(r.w) << 32;
+        red_min(&minval[r.a], w | r.b);
+        red_min(&minval[r.b], w | r.a);
+      }
+      ++k;
+    }
+    run += tot;
+  }
+}
+
 // Weight samples for pivot selection, sorted: sample i is the weight of the
 // input entry at hi64(mix64(seed + i) * m).  Both copies of an undirected
 // edge carry its weight, so sampling the directed list samples edge weights.
+// out[kSampleCount] receives the number of sampled edges whose ids lie at
+// least n / 16 apart.
 __global__ void __launch_bounds__(kSampleBlock)
-    k_sample_weights(const uint32_t* __restrict__ in_words, uint64_t m, uint64_t seed,
+    k_sample_weights(const uint32_t* __restrict__ in_words, uint64_t m, uint32_t n, uint64_t seed,
                      uint32_t* __restrict__ out) {
+  uint32_t far = 0;
   sample_sorted(
-      [&](uint32_t i) { return in_words[__umul64hi(mix64(seed + i), m) * 3 + 2]; }, out);
+      [&](uint32_t i) {
+        const uint32_t* e = in_words + __umul64hi(mix64(seed + i), m) * 3;
+        const uint32_t s = e[0], d = e[1];
+        far += (s < d ? d - s : s - d) >= n / 16 ? 1u : 0u;
+        return e[2];
+      },
+      out);
+  __shared__ uint32_t s_far;
+  if (threadIdx.x == 0) s_far = 0;
+  __syncthreads();
+  far = warp_sum(far);
+  if (lane_id() == 0) atomicAdd(&s_far, far);
+  __syncthreads();
+  if (threadIdx.x == 0) out[kSampleCount] = s_far;
 }
 
 // Same over a segmented list; prefix[s] = records in segments < s.

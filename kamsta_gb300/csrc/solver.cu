@@ -252,6 +252,22 @@ constexpr uint32_t kTailN = 1u << 23;
 // the update's gathers need the full occupancy of its own kernels.
 constexpr uint32_t kCoopFinalizeN = 1u << 22;
 
+// Plain rounds are replayed on the forest (run_sparse) for inputs of at least
+// kSparseMinMd entries with 24 or more entries per vertex, and from
+// kSparseFarMd entries on with 14 or more when most edges join far ids.
+// What decides is how many edges the rounds keep: where ids follow geometry
+// they lose a third and more each round, else most stay to the end.  All
+// edges / forest, us: degree 32, 2^20 and 2^22 vertices: G(n,m) 1599 / 1131,
+// 6555 / 2198, RGG-2D 1040 / 859, 3556 / 2049, R-MAT 961 / 889, 3553 / 2584;
+// degree 16, 2^21 and 2^22: G(n,m) 1627 / 1524, 3520 / 2543, RGG-2D 969 /
+// 1021, 1805 / 2022, R-MAT 1001 / 1060, 2185 / 2019; below 2^25 entries the
+// replay's extra launches cost as much as it saves.
+constexpr uint64_t kSparseMinMd = 1ull << 25, kSparseFarMd = 1ull << 26;
+constexpr uint64_t kSparseDegree = 24, kSparseFarDegree = 14;
+// Smallest input whose forest bitmap (batches) is found by weight classes
+// when no preprocessing was asked for.
+constexpr uint64_t kBitsClassMd = 1ull << 23;
+
 template <typename K>
 static int blocks_per_sm(K kernel, size_t dyn_smem) {
   int per_sm = 1;
@@ -337,11 +353,17 @@ class Solve {
   kamsta_status pick_big(uint32_t* label, bool* use);
   bool use_big_ = false;
   uint32_t big_label_ = 0;
-  std::vector<uint32_t> plan_classes();
+  // as_preprocessed: as if local preprocessing were requested
+  std::vector<uint32_t> plan_classes(bool as_preprocessed);
   kamsta_status sample_weights(const SegList* L, std::vector<uint32_t>* out);
   kamsta_status fetch_samples(std::vector<uint32_t>* out);
   kamsta_status filter_rec(SegList* L, bool own, bool stop, int depth);
   kamsta_status run_boruvka();
+  kamsta_status run_classes();
+  // Plain rounds over the forest's edges alone; *done = false: not worth it,
+  // or no memory for it.
+  kamsta_status run_sparse(bool* done);
+  bool sparse_ = false;  // collecting the forest for run_sparse
   // The first pass; with fetch = false its counts stay on the device.
   kamsta_status first_pass(SegList** C, int nmat, bool fetch);
   // ---- cooperative rounds (rounds_coop.cuh)
@@ -1052,7 +1074,7 @@ kamsta_status Solve::finish_rounds(const Rounds& rs, uint32_t n0) {
 // sampling and planning
 
 kamsta_status Solve::fetch_samples(std::vector<uint32_t>* out) {
-  CU_TRY(cudaMemcpyAsync(ctx_->h_samples, samples_, kSampleCount * sizeof(uint32_t),
+  CU_TRY(cudaMemcpyAsync(ctx_->h_samples, samples_, (kSampleCount + 1) * sizeof(uint32_t),
                          cudaMemcpyDeviceToHost, st_));
   CU_TRY(cudaStreamSynchronize(st_));
   out->assign(ctx_->h_samples, ctx_->h_samples + kSampleCount);
@@ -1075,7 +1097,7 @@ kamsta_status Solve::sample_weights(const SegList* L, std::vector<uint32_t>* out
                            cudaMemcpyHostToDevice, st_));
     k_sample_weights_seg<<<1, kSampleBlock, 0, st_>>>(L->in(), prefix_, m, cfg_.seed, samples_);
   } else {
-    k_sample_weights<<<1, kSampleBlock, 0, st_>>>(in_, m, cfg_.seed, samples_);
+    k_sample_weights<<<1, kSampleBlock, 0, st_>>>(in_, m, n_, cfg_.seed, samples_);
   }
   tock(KAMSTA_PHASE_PLAN, tp);
   account(KAMSTA_PHASE_PLAN, uint64_t(kSampleCount) * 8, 1);
@@ -1088,9 +1110,9 @@ kamsta_status Solve::sample_weights(const SegList* L, std::vector<uint32_t>* out
 // (local_mst_respecting_cut_edges.hpp:209-260): recurse while the level has
 // more than 3n edges and its 25%-quantile split (mst_utils_filter.hpp:13-30)
 // is balanced (mst_utils_filter.hpp:32-37).  Returned in descending order.
-std::vector<uint32_t> Solve::plan_classes() {
+std::vector<uint32_t> Solve::plan_classes(bool as_preprocessed) {
   std::vector<uint32_t> thr;
-  if (cfg_.local_preprocessing == KAMSTA_NO_PREPROCESSING) return thr;
+  if (cfg_.local_preprocessing == KAMSTA_NO_PREPROCESSING && !as_preprocessed) return thr;
   std::vector<uint32_t>& s = samples_host_;
   if (sample_weights(nullptr, &s) != KAMSTA_OK) return thr;
   double m_est = static_cast<double>(md_) / 2.0;
@@ -1102,7 +1124,7 @@ std::vector<uint32_t> Solve::plan_classes() {
   // on 1024 mixed graphs 78.6 against 86.0 ms, while single graphs are
   // fastest at 3n (GNM 2^26 deg 32 / deg 16, RGG-2D, RHG, R-MAT 2^24: 0-20%
   // slower at 2n).
-  const double stop = forest_bits_ != nullptr ? 2.0 : 3.0;
+  const double stop = forest_bits_ != nullptr && !sparse_ ? 2.0 : 3.0;
   while (m_est > stop * nv && len >= 16) {
     const uint32_t pivot = s[static_cast<size_t>(len * 0.25)];
     const size_t light =
@@ -1591,7 +1613,96 @@ kamsta_status Solve::first_pass(SegList** C, int nmat, bool fetch) {
   }
 }
 
+// Plain Boruvka rounds find the forest's edges and nothing else: the minimum
+// edge of a component is a forest edge, so rounds over the forest's edges
+// alone hook, number and emit exactly like rounds over all edges.  With many
+// edges per vertex it is cheaper to find the forest first, by weight classes
+// as local preprocessing does (each touches few edges), and to replay the
+// rounds on its n - 1 edges for the plain rounds' output order.
+kamsta_status Solve::run_sparse(bool* done) {
+  *done = false;
+  const std::vector<uint32_t> thr = plan_classes(true);
+  if (thr.empty()) return KAMSTA_OK;
+  const bool far = ctx_->h_samples[kSampleCount] >= kSampleCount / 4 * 3;
+  if (md_ < kSparseDegree * n_ && !(far && md_ >= kSparseFarMd)) return KAMSTA_OK;
+  const uint64_t words = (md_ + 31) / 32;
+  void* mem = nullptr;
+  const cudaError_t e = ctx_alloc(ctx_, &mem, words * sizeof(uint32_t), st_);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return KAMSTA_OK;
+  }
+  struct Free {
+    kamsta_ctx* c;
+    void* p;
+    cudaStream_t s;
+    ~Free() { ctx_free(c, p, s); }
+  } fm{ctx_, mem, st_};
+  uint32_t* bits = static_cast<uint32_t*>(mem);
+  CU_TRY(cudaMemsetAsync(bits, 0, words * sizeof(uint32_t), st_));
+  bounds_.assign(thr.rbegin(), thr.rend());
+  forest_bits_ = bits;
+  sparse_ = true;
+  kamsta_status s = run_classes();
+  forest_bits_ = nullptr;
+  sparse_ = false;
+  bounds_.clear();
+  SegList* E = nullptr;
+  const uint64_t k = msf_count_;
+  if (s == KAMSTA_OK) {
+    if (!coop_done_ && k > 0) {
+      k_mark_forest<<<grid_for(k), kBlock, 0, st_>>>(k, msf_, bits);
+      account(KAMSTA_PHASE_EMIT, k * 12, 1);
+    }
+    E = new_list();
+    s = alloc_list(E, 1, k);
+  }
+  // what run_classes left behind is started over
+  coop_done_ = false;
+  msf_count_ = 0;
+  nreps_ = n_;
+  rounds_ = levels_ = row_scans_ = 0;
+  for (SegList* L : owned_)
+    if (L != E) free_list(L);
+  k_init_vertices<<<grid_for(n_), kBlock, 0, st_>>>(n_, minA_, P_, V_, D_);
+  if (s == KAMSTA_E_OOM) {
+    cudaGetLastError();
+    CU_TRY(cudaMemsetAsync(ctx_->d_err, 0, sizeof(uint32_t), st_));
+    return KAMSTA_OK;
+  }
+  KS_TRY(s);
+  const int t0 = tick();
+  const uint32_t grid = static_cast<uint32_t>(
+      std::max<uint64_t>(1, std::min<uint64_t>(kMaxSeg, (words + kBlock - 1) / kBlock)));
+  const uint64_t chunk = round_up((words + grid - 1) / grid, kBlock);
+  k_bits_count<<<grid, kBlock, 0, st_>>>(bits, words, chunk, cta_counts_);
+  k_bits_list<<<grid, kBlock, 0, st_>>>(bits, words, chunk, cta_counts_, in_, E->cap, E->base,
+                                        minA_, E->d_count);
+  tock(KAMSTA_PHASE_CLASS_PASS, t0);
+  CU_TRY(cudaGetLastError());
+  account(KAMSTA_PHASE_CLASS_PASS, words * 8 + k * (12 + 16 + 16), 2);
+  E->h_count.assign(1, static_cast<uint32_t>(k));
+  E->total = k;
+  direct_emit_ = d_out_ != nullptr && n_ >= 2;
+  final_contraction_ = true;
+  const kamsta_status r = rounds(E, true);
+  direct_emit_ = final_contraction_ = false;
+  KS_TRY(r);
+  *done = true;
+  return KAMSTA_OK;
+}
+
 kamsta_status Solve::run_boruvka() {
+  if (cfg_.local_preprocessing == KAMSTA_NO_PREPROCESSING && forest_bits_ == nullptr &&
+      coop_options() && md_ >= kSparseMinMd && md_ >= kSparseFarDegree * n_) {
+    bool done = false;
+    KS_TRY(run_sparse(&done));
+    if (done) return KAMSTA_OK;
+  }
+  return run_classes();
+}
+
+kamsta_status Solve::run_classes() {
   if (coop_fits()) {
     bool done = false;
     KS_TRY(run_coop(&done));
@@ -1755,7 +1866,9 @@ kamsta_status Solve::run(Algo algo, kamsta_wedge* d_out, SolveOut* out) {
     input_complete_ = true;
   }
   if (algo == Algo::kBoruvka) {
-    std::vector<uint32_t> thr_desc = plan_classes();
+    // a bitmap of the forest does not show in what order it was found
+    const bool classes = forest_bits_ != nullptr && coop_options() && md_ >= kBitsClassMd;
+    std::vector<uint32_t> thr_desc = plan_classes(classes);
     bounds_.assign(thr_desc.rbegin(), thr_desc.rend());
   }
   k_init_vertices<<<grid_for(n_), kBlock, 0, st_>>>(n_, minA_, P_, V_, D_);

@@ -73,6 +73,7 @@ static_assert(sizeof(DevCounters) == 128, "counter block size");
 
 enum CounterSlot : int { kCVertex = 0, kCEdge = 1, kCRep = 2, kCMisc = 3, kCSlots = 4 };
 constexpr uint32_t kSampleCap = 4096;
+constexpr uint32_t kSampleWords = kSampleCap + 16;  // the sample, then its counters
 constexpr int kTimerEvents = 64;
 constexpr size_t kHostState = 1024;  // bytes of kamsta_ctx::h_state
 constexpr int kInputPieces = 16;  // host input copied in this many pieces

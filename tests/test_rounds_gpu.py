@@ -169,3 +169,45 @@ def test_scratch_heap_limits_and_trim(kamsta, oracle):
     again, k, _ = _dev_solve(kamsta, ctx, big, n, cfg)
     assert k == k0 and np.array_equal(again, first)
     ctx.close()
+
+
+@pytest.mark.parametrize("family,log_n,degree,wmax", [
+    ("gnm", 20, 33, 254), ("gnm", 22, 17, 254), ("rgg2d", 21, 33, 254), ("rmat", 21, 34, 254),
+    ("gnm", 21, 17, 254), ("rgg2d", 22, 17, 254), ("rmat", 22, 18, 254),
+    ("gnm", 20, 40, 1 << 30), ("gnm", 20, 33, 2), ("gnm", 15, 2000, 254)])
+def test_plain_rounds_replayed_on_the_forest(kamsta, family, log_n, degree, wmax):
+    """Without preprocessing a large dense input is solved on its forest's
+    edges; the output is byte for byte that of rounds over every edge (which
+    a traced solve runs), order included, with and without validation."""
+    import math
+
+    import torch
+    ctx = kamsta.Context(0)
+    n, m = (1 << log_n) - 3, int((1 << log_n) * degree / 2)
+    if family == "gnm":
+        d = torch.empty((2 * m, 3), dtype=torch.int32, device="cuda")
+        md = ctx.gen_gnm_dev(n, m, 5, wmax, d.data_ptr())
+    elif family == "rgg2d":
+        r = math.sqrt(degree / (math.pi * n))
+        md = ctx.gen_rgg2d_dev(n, r, 5, wmax)
+        d = torch.empty((md, 3), dtype=torch.int32, device="cuda")
+        ctx.gen_rgg2d_dev(n, r, 5, wmax, d.data_ptr(), md)
+    else:
+        n = 1 << log_n
+        md = ctx.gen_rmat_dev(log_n, m, 5, max_weight=wmax)
+        d = torch.empty((md, 3), dtype=torch.int32, device="cuda")
+        ctx.gen_rmat_dev(log_n, m, 5, max_weight=wmax, d_out=d.data_ptr(), capacity=md)
+    torch.cuda.synchronize()
+    o = torch.zeros((2, n, 3), dtype=torch.int32, device="cuda")
+    want, got = {}, {}
+    kw = ctx.boruvka_dev(d.data_ptr(), md, n, o[0].data_ptr(),
+                         kamsta.AlgorithmConfig(trace=True), stats=want)
+    for validate in (False, True):
+        o[1].zero_()
+        torch.cuda.synchronize()
+        k = ctx.boruvka_dev(d.data_ptr(), md, n, o[1].data_ptr(),
+                            kamsta.AlgorithmConfig(validate=validate), stats=got)
+        assert k == kw and got["total_weight"] == want["total_weight"]
+        assert got["rounds"] == want["rounds"] and got["levels"] == want["levels"] == 1
+        assert torch.equal(o[0], o[1])
+    ctx.close()
