@@ -460,6 +460,11 @@ kamsta_status kamsta_ctx_create(int device, kamsta_ctx** out) {
   kamsta_status s = KAMSTA_OK;
   if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&c->aux, cudaStreamNonBlocking)) != cudaSuccess ||
+      (e = cudaStreamCreateWithFlags(&c->small_st[0], cudaStreamNonBlocking)) != cudaSuccess ||
+      (e = cudaStreamCreateWithFlags(&c->small_st[1], cudaStreamNonBlocking)) != cudaSuccess ||
+      (e = cudaEventCreateWithFlags(&c->ev_small[0], cudaEventDisableTiming)) != cudaSuccess ||
+      (e = cudaEventCreateWithFlags(&c->ev_small[1], cudaEventDisableTiming)) != cudaSuccess ||
+      (e = cudaEventCreateWithFlags(&c->ev_small[2], cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&c->ev_early, cudaEventDisableTiming)) != cudaSuccess ||
@@ -509,6 +514,8 @@ kamsta_status kamsta_ctx_destroy(kamsta_ctx* ctx) {
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->aux) cudaStreamSynchronize(ctx->aux);
+  for (cudaStream_t s : ctx->small_st)
+    if (s) cudaStreamSynchronize(s);
   ctx->fixed.release();
   heap_release(ctx);
   if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
@@ -529,7 +536,11 @@ kamsta_status kamsta_ctx_destroy(kamsta_ctx* ctx) {
   for (int i = 0; i < kInputPieces; ++i)
     if (ctx->piece_ev[i]) cudaEventDestroy(ctx->piece_ev[i]);
   if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
+  for (cudaEvent_t e : ctx->ev_small)
+    if (e) cudaEventDestroy(e);
   if (ctx->aux) cudaStreamDestroy(ctx->aux);
+  for (cudaStream_t s : ctx->small_st)
+    if (s) cudaStreamDestroy(s);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   cudaSetDevice(prev);
   delete ctx;

@@ -399,14 +399,21 @@ std::vector<std::pair<uint32_t, uint32_t>> plan_waves(const kamsta_graph_desc* g
 namespace {
 
 // ---------------------------------------------------------------------------
-// Small graphs (n <= 32768, m_directed <= 262144): one persistent launch.
+// Small graphs (n <= 32768, m_directed <= 262144): persistent launches.
 // Each CTA takes the next graph from a work queue (largest first) and solves
 // it entirely on its own (small_solve.cuh) in its own scratch slot; the
-// forest comes out sorted by (src, dst), like the union path's.
+// forest comes out sorted by (src, dst), like the union path's.  The graphs'
+// size class picks the CTA: 128 threads (8 CTAs per SM), 512 (2) or all of an
+// SM; the classes run side by side on streams of their own.  1024 graphs of
+// 2^8..2^12 vertices, us per call: the compact class on 256, 512, 1024
+// threads 331, 322, 386.
 
-// CTA sizes the persistent kernel is built for; the context's tuning picks
-// one (kamsta_batch_autotune), 512 by default.
+// CTA sizes the compact class is built for; the context's tuning picks one
+// (kamsta_batch_autotune), 512 by default.
 constexpr int kSmallThreadsDefault = 512;
+constexpr int kTinyThreads = 128;
+constexpr int kFullThreads = 1024;
+constexpr int kClasses = 3;
 
 struct SmallTable {
   const uint32_t* const* edges;
@@ -415,15 +422,16 @@ struct SmallTable {
   const uint32_t* n;
   const uint32_t* order;  // graph indices, largest first
   small::Result* res;
-  uint32_t G;
+  uint32_t G;             // graphs in order
   uint32_t check_order;
 };
 
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS)
+template <int THREADS, small::Size CLASS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
     k_small_batch(SmallTable t, unsigned char* __restrict__ scratch, uint32_t* queue) {
+  extern __shared__ __align__(16) unsigned char s_raw[];
   __shared__ uint32_t s_q;
-  unsigned char* mine = scratch + static_cast<size_t>(blockIdx.x) * small::kScratchBytes;
+  unsigned char* mine = scratch + static_cast<size_t>(blockIdx.x) * small::slot_layout(CLASS).bytes;
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) s_q = atomicAdd(queue, 1u);
@@ -431,8 +439,8 @@ __global__ void __launch_bounds__(THREADS)
     const uint32_t q = s_q;
     if (q >= t.G) return;
     const uint32_t g = t.order[q];
-    small::solve<THREADS, small::Out::kSorted>(t.edges[g], t.md[g], t.n[g], mine, t.out[g],
-                                                      &t.res[g], true, t.check_order != 0);
+    small::solve<THREADS, small::Out::kSorted, CLASS>(t.edges[g], t.md[g], t.n[g], mine, t.out[g],
+                                                      &t.res[g], s_raw, true, t.check_order != 0);
   }
 }
 
@@ -445,35 +453,70 @@ bool is_small(const kamsta_ctx* ctx, const kamsta_graph_desc& g) {
   return g.n <= small_max_n(ctx) && g.m_directed <= small::kMaxMd;
 }
 
-template <int THREADS>
+int size_class(const kamsta_graph_desc& g) {
+  for (int c = 0; c < kClasses - 1; ++c)
+    if (g.n <= small::max_n(small::Size(c)) && g.m_directed <= small::max_md(small::Size(c)))
+      return c;
+  return kClasses - 1;
+}
+
+// Launches grid CTAs; without scratch, only asks how many fit an SM.
+template <int THREADS, small::Size CLASS>
 cudaError_t launch_small_kernel(const SmallTable& t, unsigned char* scratch, uint32_t* queue,
-                                uint32_t grid, cudaStream_t st) {
-  k_small_batch<THREADS><<<grid, THREADS, 0, st>>>(t, scratch, queue);
+                                uint32_t grid, int* per_sm, cudaStream_t st) {
+  const auto k = k_small_batch<THREADS, CLASS>;
+  const size_t smem = small::shared_bytes(CLASS);
+  if (!scratch) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem));
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, THREADS, smem);
+    *per_sm = std::max(*per_sm, 1);
+    return e;
+  }
+  k<<<grid, THREADS, smem, st>>>(t, scratch, queue);
   return cudaGetLastError();
 }
 
-int small_per_sm(int threads) {
-  int per_sm = 1;
+cudaError_t launch_small_kernel(int c, int threads, const SmallTable& t, unsigned char* scratch,
+                                uint32_t* queue, uint32_t grid, int* per_sm, cudaStream_t st) {
+  using S = small::Size;
+  if (c == 0)
+    return launch_small_kernel<kTinyThreads, S::kTiny>(t, scratch, queue, grid, per_sm, st);
+  if (c == 2)
+    return launch_small_kernel<kFullThreads, S::kFull>(t, scratch, queue, grid, per_sm, st);
   if (threads == 256)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_small_batch<256>, 256, 0);
-  else if (threads == 1024)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_small_batch<1024>, 1024, 0);
-  else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_small_batch<512>, 512, 0);
-  return std::max(per_sm, 1);
+    return launch_small_kernel<256, S::kCompact>(t, scratch, queue, grid, per_sm, st);
+  if (threads == 1024)
+    return launch_small_kernel<1024, S::kCompact>(t, scratch, queue, grid, per_sm, st);
+  return launch_small_kernel<512, S::kCompact>(t, scratch, queue, grid, per_sm, st);
 }
 
-// Launches the small graphs on `st` and returns; `res` (host) is valid after
-// the stream synchronises.  Device buffers stay alive in `keep`.
+// Launches the small graphs, each size class on a stream of its own between
+// `st` and `st`, and returns; `res` (host) is valid after st synchronises.
+// Device buffers stay alive in tab and scr.
 kamsta_status launch_small(kamsta_ctx* ctx, kamsta_graph_desc* g, const std::vector<uint32_t>& idx,
                            const kamsta_cfg& cfg, cudaStream_t st, PoolBuf* tab, PoolBuf* scr,
                            small::Result** d_res, uint32_t* launches) {
   const uint32_t S = static_cast<uint32_t>(idx.size());
-  std::vector<uint32_t> order(S);
-  for (uint32_t i = 0; i < S; ++i) order[i] = i;
-  std::sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
-    return g[idx[a]].m_directed + g[idx[a]].n > g[idx[b]].m_directed + g[idx[b]].n;
-  });
+  // by class, each by descending work to an eighth of its power of two (the
+  // queue only wants the long ones first): one counting sort
+  constexpr uint32_t kBuckets = 32 * 8;
+  std::vector<uint32_t> order(S), bucket(S);
+  uint32_t start[kClasses * kBuckets + 1] = {};
+  uint32_t count[kClasses] = {0, 0, 0};
+  for (uint32_t i = 0; i < S; ++i) {
+    const kamsta_graph_desc& d = g[idx[i]];
+    const int c = size_class(d);
+    ++count[c];
+    const uint32_t work = static_cast<uint32_t>(d.m_directed) + d.n + 8;
+    const uint32_t lg = 31u - static_cast<uint32_t>(__builtin_clz(work));
+    const uint32_t rank = lg * 8 + ((work >> (lg - 3)) & 7u);
+    bucket[i] = static_cast<uint32_t>(c) * kBuckets + (kBuckets - 1 - rank);
+    ++start[bucket[i] + 1];
+  }
+  for (int k = 0; k < kClasses * static_cast<int>(kBuckets); ++k) start[k + 1] += start[k];
+  for (uint32_t i = 0; i < S; ++i) order[start[bucket[i]]++] = i;
   const size_t o_edges = 0;
   const size_t o_out = o_edges + up256(sizeof(void*) * S);
   const size_t o_md = o_out + up256(sizeof(void*) * S);
@@ -494,38 +537,67 @@ kamsta_status launch_small(kamsta_ctx* ctx, kamsta_graph_desc* g, const std::vec
   B_TRY(tab->alloc(ctx, bytes, st));
   unsigned char* d = static_cast<unsigned char*>(tab->p);
   B_TRY(cudaMemcpyAsync(d, h.data(), bytes, cudaMemcpyHostToDevice, st));
-  int dev = 0, sms = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int sms = 1;
+  B_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   const int threads = ctx->tune_small_threads ? static_cast<int>(ctx->tune_small_threads)
                                               : kSmallThreadsDefault;
-  uint32_t grid = std::max<uint32_t>(
-      1, std::min<uint32_t>(S, static_cast<uint32_t>(small_per_sm(threads) * sms)));
-  if (ctx->mem_limit) {
-    // under a memory limit, only as many scratch slots as the limit leaves
-    // room for; the work queue spreads the graphs over however many CTAs run
-    const uint64_t used = ctx_device_bytes(ctx);
-    const uint64_t room = ctx->mem_limit > used ? ctx->mem_limit - used : 0;
-    const uint64_t slots = room / (small::kScratchBytes + 4096);
-    grid = std::max<uint32_t>(1, static_cast<uint32_t>(std::min<uint64_t>(grid, slots)));
-  }
-  B_TRY(scr->alloc(ctx, static_cast<size_t>(grid) * small::kScratchBytes, st));
   SmallTable t;
   t.edges = reinterpret_cast<const uint32_t* const*>(d + o_edges);
   t.out = reinterpret_cast<uint32_t* const*>(d + o_out);
   t.md = reinterpret_cast<const uint32_t*>(d + o_md);
   t.n = reinterpret_cast<const uint32_t*>(d + o_n);
-  t.order = reinterpret_cast<const uint32_t*>(d + o_order);
   t.res = reinterpret_cast<small::Result*>(d + o_res);
-  t.G = S;
   t.check_order = (cfg.flags & KAMSTA_FLAG_VALIDATE) ? 1u : 0u;
+  size_t slot[kClasses];
+  uint32_t grid[kClasses];
+  uint64_t room = ~0ull, least = 0;
+  for (int c = 0; c < kClasses; ++c) {
+    slot[c] = small::slot_layout(small::Size(c)).bytes;
+    grid[c] = 0;
+    if (!count[c]) continue;
+    int& per_sm = ctx->small_per_sm[c == 1 ? 1 + threads / 512 : c == 0 ? 0 : 4];
+    if (!per_sm) B_TRY(launch_small_kernel(c, threads, t, nullptr, nullptr, 0, &per_sm, st));
+    grid[c] = std::min<uint32_t>(count[c], static_cast<uint32_t>(per_sm * sms));
+    least += slot[c] + 4096;
+  }
+  if (ctx->mem_limit) {
+    // under a memory limit, only as many scratch slots as the limit leaves
+    // room for (one per class at least); the work queues spread the graphs
+    // over however many CTAs run
+    const uint64_t used = ctx_device_bytes(ctx);
+    room = ctx->mem_limit > used ? ctx->mem_limit - used : 0;
+    room = room > least ? room - least : 0;
+    for (int c = 0; c < kClasses; ++c) {
+      if (!count[c]) continue;
+      const uint64_t more = std::min<uint64_t>(grid[c] - 1, room / (slot[c] + 4096));
+      grid[c] = 1 + static_cast<uint32_t>(more);
+      room -= more * (slot[c] + 4096);
+    }
+  }
+  size_t total = 0;
+  for (int c = 0; c < kClasses; ++c) total += grid[c] * slot[c];
+  B_TRY(scr->alloc(ctx, total, st));
   unsigned char* scratch = static_cast<unsigned char*>(scr->p);
   uint32_t* queue = reinterpret_cast<uint32_t*>(d + o_queue);
-  if (threads == 256) B_TRY(launch_small_kernel<256>(t, scratch, queue, grid, st));
-  else if (threads == 1024) B_TRY(launch_small_kernel<1024>(t, scratch, queue, grid, st));
-  else B_TRY(launch_small_kernel<512>(t, scratch, queue, grid, st));
+  B_TRY(cudaEventRecord(ctx->ev_small[0], st));
+  cudaStream_t on[kClasses] = {ctx->small_st[0], ctx->small_st[1], st};
+  uint32_t first = S;
+  for (int c = kClasses - 1; c >= 0; --c) {  // the longest first
+    first -= count[c];
+    if (!count[c]) continue;
+    if (on[c] != st) B_TRY(cudaStreamWaitEvent(on[c], ctx->ev_small[0], 0));
+    t.order = reinterpret_cast<const uint32_t*>(d + o_order) + first;
+    t.G = count[c];
+    B_TRY(launch_small_kernel(c, threads, t, scratch, queue + c, grid[c], nullptr, on[c]));
+    scratch += grid[c] * slot[c];
+    ++*launches;
+  }
+  for (int c = 0; c < kClasses; ++c) {  // st goes on when all are done
+    if (!count[c] || on[c] == st) continue;
+    B_TRY(cudaEventRecord(ctx->ev_small[1 + c], on[c]));
+    B_TRY(cudaStreamWaitEvent(st, ctx->ev_small[1 + c], 0));
+  }
   *d_res = t.res;
-  ++*launches;
   return KAMSTA_OK;
 }
 
@@ -715,9 +787,6 @@ static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_de
   small::Result* d_res = nullptr;
   uint32_t launches = 0;
   B_KTRY(launch_small(ctx, g, sm, cfg, ctx->aux, &tab, &scr, &d_res, &launches));
-  std::vector<small::Result> h_res(sm.size());
-  B_TRY(cudaMemcpyAsync(h_res.data(), d_res, sizeof(small::Result) * sm.size(),
-                        cudaMemcpyDeviceToHost, ctx->aux));
   BatchWaveStats us;
   kamsta_status s = KAMSTA_OK;
   if (!lg.empty()) {
@@ -727,6 +796,11 @@ static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_de
                     st, &us);
     for (size_t k = 0; k < lg.size(); ++k) g[lg[k]] = sub[k];
   }
+  // (the copy into pageable memory waits for the small graphs, so it comes
+  // after the union solve's launches)
+  std::vector<small::Result> h_res(sm.size());
+  B_TRY(cudaMemcpyAsync(h_res.data(), d_res, sizeof(small::Result) * sm.size(),
+                        cudaMemcpyDeviceToHost, ctx->aux));
   B_TRY(cudaEventRecord(ctx->ev_join, ctx->aux));
   B_TRY(cudaStreamWaitEvent(st, ctx->ev_join, 0));
   B_TRY(cudaStreamSynchronize(ctx->aux));

@@ -27,7 +27,9 @@ namespace noalloc {
 
 constexpr uint32_t kMaxN = small::kMaxN;
 constexpr uint64_t kMaxMd = small::kMaxMd;
-constexpr int kThreads = 1024;
+// Small graphs take a smaller CTA: their phases are as short as its barriers.
+constexpr int kThreads = 1024, kThreadsFew = 256;
+constexpr uint64_t kFewMd = 1ull << 14;
 constexpr size_t kScratchBytes = small::kScratchBytes;
 using NaResult = small::Result;
 
@@ -45,11 +47,13 @@ namespace noalloc {
 // the rounds find them; the result header sits at the start of the scratch.
 // Ids are always checked against n (one compare per entry in the pass that
 // reads them anyway), so an id >= n is reported instead of skipped.
-__global__ void __launch_bounds__(kThreads, 1)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1)
     k_noalloc_boruvka(const uint32_t* __restrict__ in, uint32_t md, uint32_t n,
                       unsigned char* __restrict__ scratch, uint32_t* __restrict__ out) {
-  small::solve<kThreads, small::Out::kFound>(in, md, n, scratch, out,
-                                             reinterpret_cast<NaResult*>(scratch), true);
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  small::solve<THREADS, small::Out::kFound, small::Size::kFull>(
+      in, md, n, scratch, out, reinterpret_cast<NaResult*>(scratch), s_raw, true);
 }
 
 }  // namespace noalloc
@@ -83,6 +87,12 @@ kamsta_status scratch_for_current_device(unsigned char** out) {
     void* p = nullptr;
     e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
     if (e != cudaSuccess) return kamsta::cuda_status(e, "cudaGetSymbolAddress(scratch)");
+    using namespace kamsta::noalloc;
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const int smem = static_cast<int>(kamsta::small::kSharedFull);
+    e = cudaFuncSetAttribute(k_noalloc_boruvka<kThreads>, attr, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_noalloc_boruvka<kThreadsFew>, attr, smem);
+    if (e != cudaSuccess) return kamsta::cuda_status(e, "cudaFuncSetAttribute(k_noalloc_boruvka)");
     g_scratch_ptr[dev] = p;
   }
   *out = static_cast<unsigned char*>(g_scratch_ptr[dev]);
@@ -113,9 +123,12 @@ extern "C" kamsta_status kamsta_mst_boruvka_noalloc(const kamsta_wedge* d_edges,
   kamsta_status s = scratch_for_current_device(&scratch);
   if (s != KAMSTA_OK) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  k_noalloc_boruvka<<<1, kThreads, 0, st>>>(reinterpret_cast<const uint32_t*>(d_edges),
-                                            static_cast<uint32_t>(m_directed), n, scratch,
-                                            reinterpret_cast<uint32_t*>(d_out));
+  const uint32_t* in = reinterpret_cast<const uint32_t*>(d_edges);
+  uint32_t* out = reinterpret_cast<uint32_t*>(d_out);
+  const uint32_t md = static_cast<uint32_t>(m_directed);
+  const size_t smem = kamsta::small::shared_bytes(n);
+  if (md <= kFewMd) k_noalloc_boruvka<kThreadsFew><<<1, kThreadsFew, smem, st>>>(in, md, n, scratch, out);
+  else k_noalloc_boruvka<kThreads><<<1, kThreads, smem, st>>>(in, md, n, scratch, out);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return kamsta::cuda_status(e, "k_noalloc_boruvka launch");
   NaResult h{};

@@ -84,10 +84,14 @@ struct kamsta_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaStream_t aux = nullptr;    // second stream: small graphs of a batch wave
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t small_st[2] = {};  // size classes of those graphs beside it
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_small[3] = {};
   // batch tuning (kamsta_batch_autotune); 0 = built-in default
   uint32_t tune_small_threads = 0;  // CTA size of the persistent small-graph kernel
   uint32_t tune_small_max_n = 0;    // largest n taken by that kernel
+  // CTAs per SM of the small-graph kernels: tiny, compact by CTA size (256,
+  // 512, 1024), full; 0 = not asked yet
+  int small_per_sm[5] = {};
   // single-graph tiles (kamsta_autotune_tiles); 0 = built-in default
   uint32_t tune_dir_items = 0;      // entries per thread of the first pass
   uint32_t tune_seg_items = 0;      // records per thread of the list passes

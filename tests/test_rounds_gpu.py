@@ -211,3 +211,78 @@ def test_plain_rounds_replayed_on_the_forest(kamsta, family, log_n, degree, wmax
         assert got["rounds"] == want["rounds"] and got["levels"] == want["levels"] == 1
         assert torch.equal(o[0], o[1])
     ctx.close()
+
+
+def _noalloc(kamsta, edges, n, fill=0):
+    import ctypes as C
+
+    import torch
+    d = torch.from_numpy(edges.view(np.uint32).reshape(-1, 3).view(np.int32)).cuda()
+    o = torch.full((n, 3), fill, dtype=torch.int32, device="cuda")
+    cnt, w = C.c_uint64(0), C.c_uint64(0)
+    torch.cuda.synchronize()
+    kamsta.check(kamsta.lib().kamsta_mst_boruvka_noalloc(
+        C.c_void_p(d.data_ptr()), len(edges), n, C.c_void_p(o.data_ptr()), C.byref(cnt),
+        C.byref(w), None))
+    return o.cpu().numpy(), int(cnt.value), int(w.value)
+
+
+def _small_graphs(oracle):
+    """Around the single-CTA solver's limits: compact CTAs (4096 vertices,
+    65536 entries), labels and wide minima in shared memory (16384 vertices),
+    32-bit keys (weights against the bits of the entry count), the largest
+    graph, hubs, paths, ties, isolated vertices, a full graph."""
+    yield oracle.gen_gnm(2, 1, 1), 2
+    yield oracle.gen_gnm(300, 900, 2, 1), 300
+    for wmax in (254, 3, (1 << 16) - 2, (1 << 16) + 5, 0xffffffff):
+        yield oracle.gen_gnm(4096, 32768, 3, wmax), 4096      # 2^16 entries: 16 bits
+    yield oracle.gen_gnm(4097, 30000, 4), 4097
+    yield oracle.gen_gnm(1000, 40000, 5), 1000                # compact by n, not by entries
+    for n in (16383, 16384, 16385, 32767, 32768):
+        yield oracle.gen_gnm(n, 60000, 6), n
+        yield oracle.gen_gnm(n, 60000, 7, 1 << 30), n
+    yield oracle.gen_gnm(32768, 131072, 8, 16381), 32768      # the widest 32-bit weights
+    yield oracle.gen_gnm(32768, 131072, 9, 16385), 32768
+    yield oracle.gen_gnm(513, 513 * 256 - 257, 10), 513
+    yield oracle.gen_gnm(32768, 700, 11), 32768
+    yield oracle.symmetric_from_undirected([(i, i + 1, i + 1) for i in range(32767)]), 32768
+    yield oracle.symmetric_from_undirected([(i, i + 1, 9) for i in range(4095)]), 4096
+    yield oracle.symmetric_from_undirected([(0, i, 1 + i % 5) for i in range(1, 32768)]), 32768
+    yield oracle.gen_rgg2d(20000, oracle.rgg_radius(20000, 12), 12), 20000
+
+
+@pytest.mark.parametrize("threads", [0, 256, 512, 1024])
+def test_single_cta_solver_at_its_limits(kamsta, oracle, threads):
+    import torch
+    graphs = list(_small_graphs(oracle))
+    ctx = kamsta.Context(0)
+    ctx.set_tuning(threads, 0)
+    dev = [torch.from_numpy(e.view(np.uint32).reshape(-1, 3).view(np.int32)).cuda()
+           for e, _ in graphs]
+    outs = [torch.full((n, 3), -1, dtype=torch.int32, device="cuda") for _, n in graphs]
+    descs = (kamsta.GraphDesc * len(graphs))()
+    for d, t, o, (e, n) in zip(descs, dev, outs, graphs):
+        d.edges, d.m_directed, d.n, d.out = t.data_ptr(), len(e), n, o.data_ptr()
+    torch.cuda.synchronize()
+    ctx.batch_dev(descs)
+    torch.cuda.synchronize()
+    for d, o, (e, n) in zip(descs, outs, graphs):
+        ref, w = oracle.kruskal(e, n)
+        assert d.status == 0 and d.out_count == len(ref) and d.total_weight == w
+        got = o[: len(ref)].cpu().numpy().view(np.uint32).reshape(-1).view(kamsta.WEDGE)
+        key = (got["src"].astype(np.uint64) << np.uint64(32)) | got["dst"]
+        assert np.all(np.diff(key.astype(np.int64)) > 0)  # sorted by (src, dst)
+        assert np.array_equal(oracle.canon_keys(got), oracle.canon_keys(ref))
+        assert np.array_equal(np.sort(got["w"]), np.sort(ref["w"]))
+    ctx.close()
+
+
+def test_allocation_free_solve_writes_what_the_rounds_write(kamsta, oracle):
+    """Same order as the device entry point's plain rounds, byte for byte."""
+    ctx = kamsta.Context(0)
+    for e, n in _small_graphs(oracle):
+        want, kw, st = _dev_solve(kamsta, ctx, e, n, kamsta.AlgorithmConfig(trace=True))
+        got, k, w = _noalloc(kamsta, e, n)
+        assert k == kw and w == st["total_weight"]
+        assert np.array_equal(got, want)
+    ctx.close()
