@@ -320,7 +320,12 @@ constexpr size_t dir_dyn_smem(int items) { return 2ull * dir_tile(items) * 3 * s
 constexpr uint32_t kDirTile = dir_tile(kItemsDir);
 constexpr size_t kDirDynSmem = dir_dyn_smem(kItemsDir);
 
-template <int NOUT, int ITEMS = kItemsDir, bool MAPPED = false>
+// HUB (unmapped): a tile inside one row -- a hub's -- folds its minimum per
+// thread and warp, one reduction per warp, where every entry's own would
+// queue up on the row's one word.  R-MAT 2^22, degree 16: 342 -> 240 us.  A
+// variant of its own, for inputs whose sample finds long rows: the test alone
+// cost G(n,m) 2^26/2^30 0.2 to 0.7 of 6.1 ms.
+template <int NOUT, int ITEMS = kItemsDir, bool MAPPED = false, bool HUB = false>
 __global__ void __launch_bounds__(kBlock, ITEMS <= 8 ? 4 : 3)
     k_pass_dir(const uint32_t* __restrict__ in, PassArgs p) {
   constexpr uint32_t kDirTile = dir_tile(ITEMS);
@@ -399,6 +404,28 @@ __global__ void __launch_bounds__(kBlock, ITEMS <= 8 ? 4 : 3)
     }
     uint8_t cls[kItemsDir];
     if constexpr (!MAPPED) {  // original ids: no label reads
+      const bool hub = HUB && p.min_partner && words[0] == words[3 * (cnt - 1)];
+      if (hub) {
+        const uint32_t row = words[0];
+        uint64_t mn = kInf64;
+#pragma unroll
+        for (int j = 0; j < kItemsDir; ++j) {
+          const uint32_t t = j * kBlock + threadIdx.x;
+          const uint32_t s = words[3 * t], d = words[3 * t + 1], wt = words[3 * t + 2];
+          if (t >= cnt || s == d || s >= p.n || d >= p.n || wt < p.wmin || wt > p.wmax ||
+              weight_class<NOUT>(wt, p) != 0)
+            continue;
+          const uint64_t key = (static_cast<uint64_t>(wt) << 32) | d;
+          if (s == row) mn = key < mn ? key : mn;
+          else red_min(&p.minval[s], key);  // (unsorted input)
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const uint64_t y = __shfl_xor_sync(kFull, mn, o);
+          mn = y < mn ? y : mn;
+        }
+        if (lane_id() == 0 && mn != kInf64) red_min(&p.minval[row], mn);
+      }
 #pragma unroll
       for (int j = 0; j < kItemsDir; ++j) {
         const uint32_t t = j * kBlock + threadIdx.x;
@@ -408,7 +435,7 @@ __global__ void __launch_bounds__(kBlock, ITEMS <= 8 ? 4 : 3)
         const bool in_w = wt >= p.wmin && wt <= p.wmax;
         // partner keys: every copy feeds its own row's minimum, so a
         // tile's updates go to a few consecutive addresses
-        if (p.min_partner && in_w && weight_class<NOUT>(wt, p) == 0)
+        if (p.min_partner && !hub && in_w && weight_class<NOUT>(wt, p) == 0)
           red_min(&p.minval[s], (static_cast<uint64_t>(wt) << 32) | d);
         if (!(s < d) || !in_w) continue;
         cls[j] = weight_class<NOUT>(wt, p);
@@ -1768,26 +1795,34 @@ __global__ void __launch_bounds__(kBlock)
 // input entry at hi64(mix64(seed + i) * m).  Both copies of an undirected
 // edge carry its weight, so sampling the directed list samples edge weights.
 // out[kSampleCount] receives the number of sampled edges whose ids lie at
-// least n / 16 apart.
+// least n / 16 apart, the word after it those whose row goes on for at least
+// kLongRow entries.
+constexpr uint32_t kLongRow = 2 * kDirTile;
 __global__ void __launch_bounds__(kSampleBlock)
     k_sample_weights(const uint32_t* __restrict__ in_words, uint64_t m, uint32_t n, uint64_t seed,
                      uint32_t* __restrict__ out) {
-  uint32_t far = 0;
+  uint32_t far = 0, row = 0;
   sample_sorted(
       [&](uint32_t i) {
-        const uint32_t* e = in_words + __umul64hi(mix64(seed + i), m) * 3;
+        const uint64_t pos = __umul64hi(mix64(seed + i), m);
+        const uint32_t* e = in_words + pos * 3;
         const uint32_t s = e[0], d = e[1];
         far += (s < d ? d - s : s - d) >= n / 16 ? 1u : 0u;
+        row += pos + kLongRow < m && e[3 * kLongRow] == s ? 1u : 0u;
         return e[2];
       },
       out);
-  __shared__ uint32_t s_far;
-  if (threadIdx.x == 0) s_far = 0;
+  __shared__ uint32_t s_cnt[2];
+  if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
   __syncthreads();
   far = warp_sum(far);
-  if (lane_id() == 0) atomicAdd(&s_far, far);
+  row = warp_sum(row);
+  if (lane_id() == 0) {
+    atomicAdd(&s_cnt[0], far);
+    atomicAdd(&s_cnt[1], row);
+  }
   __syncthreads();
-  if (threadIdx.x == 0) out[kSampleCount] = s_far;
+  if (threadIdx.x < 2) out[kSampleCount + threadIdx.x] = s_cnt[threadIdx.x];
 }
 
 // Same over a segmented list; prefix[s] = records in segments < s.

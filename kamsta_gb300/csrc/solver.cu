@@ -363,6 +363,7 @@ class Solve {
   // Plain rounds over the forest's edges alone; *done = false: not worth it,
   // or no memory for it.
   kamsta_status run_sparse(bool* done);
+  bool long_rows_ = false;  // a hundredth of the input or more lies in long rows
   bool sparse_ = false;  // collecting the forest for run_sparse
   // The first pass; with fetch = false its counts stay on the device.
   kamsta_status first_pass(SegList** C, int nmat, bool fetch);
@@ -674,6 +675,7 @@ kamsta_status Solve::pass(int phase, const SegList* src, const uint32_t* map, ui
   const size_t dyn = dir ? dir_dyn_smem(items)
                          : rec_dyn_smem(sitems) + round_up(size_t(smin_n) * 8, 16);
   const bool mapped = map != nullptr;
+  const bool hub = dir && !mapped && items == 6 && long_rows_ && direct_emit_;
   const int per_sm =
       !dir ? (sitems == 2 ? blocks_per_sm(k_pass_seg<NOUT, 2>, dyn)
               : sitems == 4 ? blocks_per_sm(k_pass_seg<NOUT, 4>, dyn)
@@ -738,7 +740,8 @@ kamsta_status Solve::pass(int phase, const SegList* src, const uint32_t* map, ui
         if (b1 <= b0) continue;
         KS_TRY(wait_input(k));
         a.cta_base = b0;
-        if (items == 8) k_pass_dir<NOUT, 8, false><<<b1 - b0, kBlock, dyn, st_>>>(in_, a);
+        if (hub) k_pass_dir<NOUT, 6, false, true><<<b1 - b0, kBlock, dyn, st_>>>(in_, a);
+        else if (items == 8) k_pass_dir<NOUT, 8, false><<<b1 - b0, kBlock, dyn, st_>>>(in_, a);
         else if (items == 6) k_pass_dir<NOUT, 6, false><<<b1 - b0, kBlock, dyn, st_>>>(in_, a);
         else k_pass_dir<NOUT, 12, false><<<b1 - b0, kBlock, dyn, st_>>>(in_, a);
         b0 = b1;
@@ -759,6 +762,8 @@ kamsta_status Solve::pass(int phase, const SegList* src, const uint32_t* map, ui
       k_pass_dir<NOUT, 6, true><<<G, kBlock, dyn, st_>>>(in_, a);
     else if (dir && mapped)
       k_pass_dir<NOUT, 12, true><<<G, kBlock, dyn, st_>>>(in_, a);
+    else if (hub)
+      k_pass_dir<NOUT, 6, false, true><<<G, kBlock, dyn, st_>>>(in_, a);
     else if (dir && items == 8)
       k_pass_dir<NOUT, 8, false><<<G, kBlock, dyn, st_>>>(in_, a);
     else if (dir && items == 6)
@@ -1074,7 +1079,7 @@ kamsta_status Solve::finish_rounds(const Rounds& rs, uint32_t n0) {
 // sampling and planning
 
 kamsta_status Solve::fetch_samples(std::vector<uint32_t>* out) {
-  CU_TRY(cudaMemcpyAsync(ctx_->h_samples, samples_, (kSampleCount + 1) * sizeof(uint32_t),
+  CU_TRY(cudaMemcpyAsync(ctx_->h_samples, samples_, (kSampleCount + 2) * sizeof(uint32_t),
                          cudaMemcpyDeviceToHost, st_));
   CU_TRY(cudaStreamSynchronize(st_));
   out->assign(ctx_->h_samples, ctx_->h_samples + kSampleCount);
@@ -1115,6 +1120,7 @@ std::vector<uint32_t> Solve::plan_classes(bool as_preprocessed) {
   if (cfg_.local_preprocessing == KAMSTA_NO_PREPROCESSING && !as_preprocessed) return thr;
   std::vector<uint32_t>& s = samples_host_;
   if (sample_weights(nullptr, &s) != KAMSTA_OK) return thr;
+  long_rows_ = ctx_->h_samples[kSampleCount + 1] >= kSampleCount / 100;
   double m_est = static_cast<double>(md_) / 2.0;
   const double nv = static_cast<double>(n_);
   size_t len = s.size();
@@ -1828,6 +1834,9 @@ kamsta_status Solve::run(Algo algo, kamsta_wedge* d_out, SolveOut* out) {
     KAMSTA_DIR_ATTR(1, 6, false, d6);
     KAMSTA_DIR_ATTR(2, 6, false, d6);
     KAMSTA_DIR_ATTR(3, 6, false, d6);
+    CU_TRY(cudaFuncSetAttribute(k_pass_dir<1, 6, false, true>, attr, d6));
+    CU_TRY(cudaFuncSetAttribute(k_pass_dir<2, 6, false, true>, attr, d6));
+    CU_TRY(cudaFuncSetAttribute(k_pass_dir<3, 6, false, true>, attr, d6));
     KAMSTA_DIR_ATTR(1, 8, true, d8);
     KAMSTA_DIR_ATTR(2, 8, true, d8);
     KAMSTA_DIR_ATTR(3, 8, true, d8);

@@ -286,3 +286,28 @@ def test_allocation_free_solve_writes_what_the_rounds_write(kamsta, oracle):
         assert k == kw and w == st["total_weight"]
         assert np.array_equal(got, want)
     ctx.close()
+
+
+@pytest.mark.parametrize("hub,lp", [(3071, 1), (3073, 1), (40000, 1), (200000, 1)])
+def test_long_rows_fold_their_minimum(kamsta, oracle, hub, lp):
+    """Rows around and far beyond two tiles of the first pass, first and last
+    in the input, beside ordinary ones."""
+    rng = np.random.default_rng(hub)
+    n = hub + 20000
+    und = {}
+    for h in (0, n - 1):
+        for v in rng.choice(np.arange(1, n - 1), hub - 1, replace=False):
+            und[(min(h, int(v)), max(h, int(v)))] = int(rng.integers(1, 255))
+    for a, b in rng.integers(1, n - 1, (40000, 2)):
+        if a != b:
+            und[(min(int(a), int(b)), max(int(a), int(b)))] = int(rng.integers(1, 255))
+    e = oracle.symmetric_from_undirected([(a, b, w) for (a, b), w in sorted(und.items())])
+    ctx = kamsta.Context(0)
+    for shift in (0, 1):
+        got, k, st = _dev_solve(kamsta, ctx, e, n,
+                                kamsta.AlgorithmConfig(local_preprocessing=lp), shift=shift)
+        ref, w = oracle.kruskal(e, n)
+        f = got[:k].view(np.uint32).reshape(-1).view(kamsta.WEDGE)
+        assert st["total_weight"] == w
+        assert np.array_equal(oracle.canon_keys(f), oracle.canon_keys(ref))
+    ctx.close()
