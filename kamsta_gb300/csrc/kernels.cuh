@@ -1324,27 +1324,70 @@ __global__ void k_big_bitmap(uint32_t n, const uint32_t* __restrict__ D, uint32_
 // outside vertices -- the input is (src, dst)-sorted, so a row is one
 // search away -- instead of streaming the whole input.  A record carries
 // the position of either copy of its edge (the emit writes (min, max, w)
-// whichever it is) and a key (min id << b | max id); sorting by the key
-// restores the streaming pass's order, which is the order of the src < dst
-// copies.  With `canon` set (the batch's forest bitmap, which needs the
-// src < dst copy's position) the position of that copy is searched for.
+// whichever it is).  With `canon` set (the batch's forest bitmap, which needs
+// the src < dst copy's position) the position of that copy is searched for.
+//
+// The records have to end up in the streaming pass's order, which is the
+// order of the src < dst copies: by (min id, max id).  The outside vertices
+// are listed in ascending order and the records written in row order behind
+// one another (counts, a scan, then the write), so one stable sort by the min
+// id alone restores it: a min id outside the component has its records from
+// its own row, by max id; one inside has one record from each outside row,
+// and those rows come in the order of their vertices, the max ids.
+//
+// RGG-2D 2^24 (0.5 M outside rows, 3.7 M records), us, before -> now: finding
+// and counting rows 638 -> 92 (one warp per row searched 32-way; the search
+// is a chain of dependent reads, so now each thread runs its own, with every
+// chain of the SM in flight), writing 297 -> 52, sorting 437 -> 213 (six
+// digits of (min, max) -> three of min).
 
-// Vertices outside the largest component (bit 0 in `big`), any order; one
-// counter atomic per warp and step.
-__global__ void k_outside_big(uint32_t n, const uint32_t* __restrict__ big, uint32_t* __restrict__ out,
-                             uint32_t cap, unsigned long long* count) {
-  const uint32_t words = (n + 31) / 32;
-  const uint32_t lane = lane_id();
-  const uint32_t stride = gridDim.x * blockDim.x;
-  const uint32_t start = blockIdx.x * blockDim.x + threadIdx.x;
-  for (uint32_t w0 = start - lane; w0 < words; w0 += stride) {  // warp-uniform loop
-    const uint32_t wi = w0 + lane;
-    uint32_t f = 0;
-    const uint32_t base = wi * 32;
-    if (wi < words) {
-      f = ~big[wi];
-      if (base + 32 > n) f &= (n - base >= 32) ? ~0u : ((1u << (n - base)) - 1);
-    }
+// Vertices outside the largest component (bit 0 in `big`) in ascending order:
+// k_outside_count counts each CTA's words, k_outside_write places its
+// vertices behind those of the CTAs before it.
+__device__ __forceinline__ uint32_t outside_word(uint32_t n, const uint32_t* big, uint32_t wi) {
+  const uint32_t base = wi * 32;
+  if (base >= n) return 0;
+  const uint32_t f = ~big[wi];
+  return n - base >= 32 ? f : f & ((1u << (n - base)) - 1);
+}
+__global__ void __launch_bounds__(kBlock)
+    k_outside_count(uint32_t n, const uint32_t* __restrict__ big, uint32_t chunk,
+                    uint32_t* __restrict__ cta_counts, unsigned long long* total) {
+  const uint32_t lo = blockIdx.x * chunk;
+  uint32_t c = 0;
+  for (uint32_t q = threadIdx.x; q < chunk; q += kBlock) c += __popc(outside_word(n, big, lo + q));
+  __shared__ uint32_t s_c;
+  if (threadIdx.x == 0) s_c = 0;
+  __syncthreads();
+  c = warp_sum(c);
+  if (lane_id() == 0 && c) atomicAdd(&s_c, c);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    cta_counts[blockIdx.x] = s_c;
+    if (s_c) atomicAdd(total, static_cast<unsigned long long>(s_c));
+  }
+}
+__global__ void __launch_bounds__(kBlock)
+    k_outside_write(uint32_t n, const uint32_t* __restrict__ big, uint32_t chunk,
+                    const uint32_t* __restrict__ cta_counts, uint32_t* __restrict__ out,
+                    uint32_t cap) {
+  constexpr int kWarps = kBlock / 32;
+  __shared__ uint32_t s_w[2][kWarps];
+  __shared__ uint32_t s_base;
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  if (threadIdx.x < 32) {
+    uint32_t b = 0;
+    for (uint32_t c = threadIdx.x; c < blockIdx.x; c += 32) b += cta_counts[c];
+    b = warp_sum(b);
+    if (threadIdx.x == 0) s_base = b;
+  }
+  __syncthreads();
+  uint32_t run = s_base;
+  const uint32_t lo = blockIdx.x * chunk;
+  int flip = 0;
+  for (uint32_t q0 = 0; q0 < chunk; q0 += kBlock, flip ^= 1) {
+    const uint32_t wi = lo + q0 + threadIdx.x;
+    uint32_t f = q0 + threadIdx.x < chunk ? outside_word(n, big, wi) : 0u;
     const uint32_t c = __popc(f);
     uint32_t incl = c;
 #pragma unroll
@@ -1352,22 +1395,25 @@ __global__ void k_outside_big(uint32_t n, const uint32_t* __restrict__ big, uint
       const uint32_t y = __shfl_up_sync(kFull, incl, o);
       if (lane >= static_cast<uint32_t>(o)) incl += y;
     }
-    unsigned long long wbase = 0;
-    if (lane == 31 && incl) wbase = atomicAdd(count, static_cast<unsigned long long>(incl));
-    wbase = __shfl_sync(kFull, wbase, 31);
-    uint64_t k = wbase + incl - c;
-    while (f) {
-      const uint32_t b = __ffs(f) - 1;
-      f &= f - 1;
-      if (k < cap) out[k] = base + b;
-      ++k;
+    if (lane == 31) s_w[flip][warp] = incl;
+    __syncthreads();
+    uint32_t pre = 0, tot = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const uint32_t x = s_w[flip][w];
+      if (static_cast<uint32_t>(w) < warp) pre += x;
+      tot += x;
     }
+    uint32_t k = run + pre + incl - c;
+    for (; f; f &= f - 1, ++k)
+      if (k < cap) out[k] = wi * 32 + (__ffs(f) - 1);
+    run += tot;
   }
 }
 
 // Fence index of the (src, dst)-sorted input: fence[i] = src of entry
-// i * kFenceStep (i < ceil(md / kFenceStep)).  A row search then runs on the
-// fences (a few MB, L2-resident) and then inside one kFenceStep window.
+// i * kFenceStep (i < ceil(md / kFenceStep)).  A row search runs on the fences
+// (a few MB, L2-resident) and then inside one kFenceStep window.
 constexpr uint32_t kFenceStep = 1024;
 __global__ void k_fences(const uint32_t* __restrict__ in, uint64_t md, uint32_t* __restrict__ fence) {
   const uint64_t nf = (md + kFenceStep - 1) / kFenceStep;
@@ -1376,11 +1422,17 @@ __global__ void k_fences(const uint32_t* __restrict__ in, uint64_t md, uint32_t*
     fence[i] = in[3 * i * kFenceStep];
 }
 
-// first directed entry with src >= v (entries [0, md) sorted by src); one
-// thread
+// first directed entry with src >= v (entries [0, md) sorted by src)
 __device__ __forceinline__ uint64_t row_begin(const uint32_t* __restrict__ in, uint64_t md,
-                                              uint32_t v) {
-  uint64_t lo = 0, hi = md;
+                                              const uint32_t* __restrict__ fence, uint32_t v) {
+  uint64_t lo = 0, hi = (md + kFenceStep - 1) / kFenceStep;
+  while (lo < hi) {  // first fence with src >= v
+    const uint64_t mid = (lo + hi) >> 1;
+    if (fence[mid] < v) lo = mid + 1; else hi = mid;
+  }
+  // the answer lies in ((f - 1) step, f step]
+  hi = lo * kFenceStep < md ? lo * kFenceStep : md;
+  lo = lo == 0 ? 0 : (lo - 1) * kFenceStep;
   while (lo < hi) {
     const uint64_t mid = (lo + hi) >> 1;
     if (in[3 * mid] < v) lo = mid + 1; else hi = mid;
@@ -1388,129 +1440,123 @@ __device__ __forceinline__ uint64_t row_begin(const uint32_t* __restrict__ in, u
   return lo;
 }
 
-// The same with the whole warp: 32 probes per step shrink the range 33-fold.
-// The fences narrow the range to one kFenceStep window first (their steps
-// hit L2), so only two steps read the input.  Called by all 32 lanes with
-// the same v; every lane returns the answer.
-__device__ __forceinline__ uint64_t row_begin_warp(const uint32_t* __restrict__ in, uint64_t md,
-                                                   const uint32_t* __restrict__ fence,
-                                                   uint32_t v) {
-  const uint32_t lane = lane_id();
-  uint64_t lo = 0, hi = md;  // the answer lies in [lo, hi]
-  {
-    // first fence with src >= v: the answer lies in ((f - 1) step, f step]
-    const uint64_t nf = (md + kFenceStep - 1) / kFenceStep;
-    uint64_t flo = 0, fhi = nf;
-    while (fhi - flo > 32) {
-      const uint64_t span = fhi - flo;
-      const uint64_t p = flo + span * (lane + 1) / 33;
-      const uint32_t c = __popc(__ballot_sync(kFull, fence[p] < v));
-      const uint64_t below = __shfl_sync(kFull, p, c == 0 ? 0 : c - 1);
-      const uint64_t above = __shfl_sync(kFull, p, c == 32 ? 31 : c);
-      if (c == 0) fhi = above;
-      else if (c == 32) flo = below + 1;
-      else {
-        flo = below + 1;
-        fhi = above;
-      }
+// The rows [row_lo, row_hi) of the listed vertices, one thread each.  The end
+// is found by doubling steps from the start (rows are short against the input).
+__global__ void k_row_find(const uint32_t* __restrict__ in, uint64_t md,
+                           const uint32_t* __restrict__ fence, const uint32_t* __restrict__ S,
+                           uint32_t ns, uint32_t* __restrict__ row_lo,
+                           uint32_t* __restrict__ row_hi) {
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < ns; k += gridDim.x * blockDim.x) {
+    const uint32_t v = S[k];
+    const uint64_t a = row_begin(in, md, fence, v);
+    uint64_t lo = a, step = 16;  // entries before lo are the row's or earlier
+    while (lo + step <= md && in[3 * (lo + step - 1)] == v) {
+      lo += step;
+      step *= 2;
     }
-    const uint64_t q = flo + lane;
-    const uint64_t f = flo + __popc(__ballot_sync(kFull, q < fhi && fence[q] < v));
-    lo = f == 0 ? 0 : (f - 1) * kFenceStep;
-    hi = f * kFenceStep < md ? f * kFenceStep : md;
-  }
-  while (hi - lo > 32) {
-    const uint64_t span = hi - lo;
-    const uint64_t p = lo + span * (lane + 1) / 33;  // in [lo, hi), increasing in lane
-    const uint32_t c = __popc(__ballot_sync(kFull, in[3 * p] < v));  // a prefix of lanes
-    const uint64_t below = __shfl_sync(kFull, p, c == 0 ? 0 : c - 1);
-    const uint64_t above = __shfl_sync(kFull, p, c == 32 ? 31 : c);
-    if (c == 0) hi = above;
-    else if (c == 32) lo = below + 1;
-    else {
-      lo = below + 1;
-      hi = above;
+    uint64_t hi = lo + step < md ? lo + step : md;
+    while (lo < hi) {
+      const uint64_t mid = (lo + hi) >> 1;
+      if (in[3 * mid] <= v) lo = mid + 1; else hi = mid;
     }
+    row_lo[k] = static_cast<uint32_t>(a);
+    row_hi[k] = static_cast<uint32_t>(lo);
   }
-  const uint64_t q = lo + lane;
-  const bool less = q < hi && in[3 * q] < v;
-  return lo + __popc(__ballot_sync(kFull, less));
 }
 
-// One warp per outside vertex v: every entry (v, d, w) of its row with w in
-// [wmin, wmax] whose relabelled endpoints differ; d outside too and d < v:
-// reported from d's row.  WRITE = false counts and stores each row's start
-// in row_lo; WRITE = true writes records and keys at atomic slots.
+// Surviving edges of the listed vertices' rows: every entry (v, d, w) with w
+// in [wmin, wmax] whose relabelled endpoints differ; d outside too and d < v:
+// left to d's row.  WRITE = false counts them per row into pos, WRITE = true
+// writes records and keys (the min id) from pos on.  kRowLanes lanes take a
+// row; a row longer than kRowLong the whole warp.
+constexpr uint32_t kRowLanes = 8, kRowLong = 256;
 template <bool WRITE>
-__global__ void k_row_scan(const uint32_t* __restrict__ in, uint64_t md, uint32_t n,
-                           const uint32_t* __restrict__ S, uint32_t ns, uint32_t* __restrict__ row_lo,
-                           const uint32_t* __restrict__ fence,
-                           const uint32_t* __restrict__ D, const uint32_t* __restrict__ big,
-                           uint32_t big_label, uint32_t wmin, uint32_t wmax, uint32_t canon,
-                           uint32_t key_bits, Rec* __restrict__ out, uint64_t* __restrict__ keys,
-                           uint64_t cap, unsigned long long* count, uint32_t* err) {
-  const uint32_t lane = lane_id();
+__global__ void __launch_bounds__(kBlock)
+    k_row_scan(const uint32_t* __restrict__ in, uint64_t md, uint32_t n,
+               const uint32_t* __restrict__ S, uint32_t ns, const uint32_t* __restrict__ row_lo,
+               const uint32_t* __restrict__ row_hi, uint32_t* __restrict__ pos,
+               const uint32_t* __restrict__ fence, const uint32_t* __restrict__ D,
+               const uint32_t* __restrict__ big, uint32_t big_label, uint32_t wmin, uint32_t wmax,
+               uint32_t canon, Rec* __restrict__ out, uint64_t* __restrict__ keys, uint64_t cap,
+               uint32_t* err) {
+  const uint32_t lane = lane_id(), grp = lane / kRowLanes, gl = lane % kRowLanes;
+  const uint32_t lt = lanemask_lt(), gmask = ((1u << kRowLanes) - 1) << (grp * kRowLanes);
+  constexpr uint32_t kRows = 32 / kRowLanes;  // rows per warp and step
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < ns; k += warps) {
-    const uint32_t v = S[k];
-    uint64_t lo;
+  // entry i of v's row (label la): kept?  its record (and key) in r / key
+  auto look = [&](uint32_t i, uint32_t v, uint32_t la, Rec& r, uint64_t& key) -> bool {
+    const uint32_t d = in[3ull * i + 1], w = in[3ull * i + 2];
+    if (d >= n || d == v || w < wmin || w > wmax) return false;
+    const bool d_big = (__ldg(big + (d >> 5)) >> (d & 31)) & 1u;
+    if (d < v && !d_big) return false;
+    const uint32_t lb = d_big ? big_label : D[d];
+    if (la == lb) return false;
     if (WRITE) {
-      lo = row_lo[k];
-    } else {
-      lo = row_begin_warp(in, md, fence, v);
-      if (lane == 0) row_lo[k] = static_cast<uint32_t>(lo);
+      r = v < d ? Rec{la, lb, w, i} : Rec{lb, la, w, i};
+      key = v < d ? v : d;
+      if (canon && d < v) {
+        // the src<dst copy (d, v) sits in d's row, sorted by dst
+        uint64_t a = row_begin(in, md, fence, d), b = row_begin(in, md, fence, d + 1);
+        while (a < b) {
+          const uint64_t mid = (a + b) >> 1;
+          if (in[3 * mid + 1] < v) a = mid + 1; else b = mid;
+        }
+        if (a < md && in[3 * a] == d && in[3 * a + 1] == v) r.oid = static_cast<uint32_t>(a);
+        else atomicOr(err, kErrRange);  // the input lacks (d, v)
+      }
     }
-    const uint32_t la = D[v];
-    for (uint64_t i0 = lo;; i0 += 32) {
-      const uint64_t i = i0 + lane;
-      const bool in_row = i < md && in[3 * i] == v;  // a prefix of lanes
-      if (!__any_sync(kFull, in_row)) break;
-      bool keep = false;
+    return true;
+  };
+  auto put = [&](uint64_t slot, const Rec& r, uint64_t key) {
+    if (slot < cap) {
+      out[slot] = r;
+      keys[slot] = key;
+    } else {
+      atomicOr(err, kErrOverflow);
+    }
+  };
+  for (uint32_t k0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kRows; k0 < ns;
+       k0 += warps * kRows) {
+    const uint32_t k = k0 + grp;
+    uint32_t v = 0, lo = 0, hi = 0, la = 0, at = 0;
+    if (k < ns) {
+      v = S[k];
+      lo = row_lo[k];
+      hi = row_hi[k];
+      la = D[v];
+      if (WRITE) at = pos[k];
+    }
+    const bool is_long = hi - lo > kRowLong;
+    const uint32_t steps =
+        __reduce_max_sync(kFull, is_long ? 0u : (hi - lo + kRowLanes - 1) / kRowLanes);
+    uint32_t c = 0;
+    for (uint32_t t = 0; t < steps; ++t) {
+      const uint32_t o = t * kRowLanes + gl;
       Rec r;
       uint64_t key = 0;
-      if (in_row) {
-        const uint32_t d = in[3 * i + 1], w = in[3 * i + 2];
-        if (d < n && d != v && w >= wmin && w <= wmax) {
-          const bool d_big = (__ldg(big + (d >> 5)) >> (d & 31)) & 1u;
-          const uint32_t lb = d_big ? big_label : D[d];
-          if (la != lb) {
-            if (v < d) {
-              keep = true;
-              r = Rec{la, lb, w, static_cast<uint32_t>(i)};
-              key = (static_cast<uint64_t>(v) << key_bits) | d;
-            } else if (d_big) {
-              keep = true;
-              r = Rec{lb, la, w, static_cast<uint32_t>(i)};
-              key = (static_cast<uint64_t>(d) << key_bits) | v;
-              if (WRITE && canon) {
-                // the src<dst copy (d, v) sits in d's row, sorted by dst
-                uint64_t a = row_begin(in, md, d), b = row_begin(in, md, d + 1);
-                while (a < b) {
-                  const uint64_t mid = (a + b) >> 1;
-                  if (in[3 * mid + 1] < v) a = mid + 1; else b = mid;
-                }
-                if (a < md && in[3 * a] == d && in[3 * a + 1] == v) r.oid = static_cast<uint32_t>(a);
-                else atomicOr(err, kErrRange);  // the input lacks (d, v)
-              }
-            }
-          }
-        }
-      }
-      const uint32_t bal = __ballot_sync(kFull, keep);
-      if (!bal) continue;
-      unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(count, static_cast<unsigned long long>(__popc(bal)));
-      base = __shfl_sync(kFull, base, 0);
-      if (WRITE && keep) {
-        const uint64_t slot = base + __popc(bal & lanemask_lt());
-        if (slot < cap) {
-          out[slot] = r;
-          keys[slot] = key;
-        } else {
-          atomicOr(err, kErrOverflow);
-        }
-      }
+      const bool keep = !is_long && o < hi - lo && look(lo + o, v, la, r, key);
+      const uint32_t bal = __ballot_sync(kFull, keep) & gmask;
+      if (WRITE && keep) put(uint64_t(at) + c + __popc(bal & lt), r, key);
+      c += __popc(bal);
     }
+    for (uint32_t longs = __ballot_sync(kFull, is_long && gl == 0); longs; longs &= longs - 1) {
+      const uint32_t src = __ffs(longs) - 1;
+      const uint32_t lv = __shfl_sync(kFull, v, src), llo = __shfl_sync(kFull, lo, src),
+                     lhi = __shfl_sync(kFull, hi, src), lla = __shfl_sync(kFull, la, src),
+                     lat = __shfl_sync(kFull, at, src);
+      uint32_t lc = 0;
+      for (uint64_t i0 = llo; i0 < lhi; i0 += 32) {
+        Rec r;
+        uint64_t key = 0;
+        const bool keep =
+            i0 + lane < lhi && look(static_cast<uint32_t>(i0 + lane), lv, lla, r, key);
+        const uint32_t bal = __ballot_sync(kFull, keep);
+        if (WRITE && keep) put(uint64_t(lat) + lc + __popc(bal & lt), r, key);
+        lc += __popc(bal);
+      }
+      if (src / kRowLanes == grp) c = lc;
+    }
+    if (!WRITE && k < ns && gl == 0) pos[k] = c;
   }
 }
 

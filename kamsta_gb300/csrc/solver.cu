@@ -1184,41 +1184,66 @@ kamsta_status Solve::contract_rows(uint32_t wmin, uint32_t wmax, SegList* E, boo
   *done = false;
   // the vertices outside the largest component
   const uint32_t cap_s = std::max<uint32_t>(1u << 16, n_ / 32);
-  // outside vertices, their row starts, then the input's fence index
+  // outside vertices, their rows and record counts, the input's fence index
   const uint64_t nfence = (md_ + kFenceStep - 1) / kFenceStep;
+  const size_t scan_words = cap_s / 2048 + 2;  // exclusive_scan_u32's status
   void* smem = nullptr;
-  CU_TRY(ctx_alloc(ctx_, &smem, sizeof(uint32_t) * (2 * uint64_t(cap_s) + nfence + 1), st_));
+  const cudaError_t ea =
+      ctx_alloc(ctx_, &smem, sizeof(uint64_t) * scan_words +
+                                 sizeof(uint32_t) * (4 * uint64_t(cap_s) + nfence + 1), st_);
+  if (ea == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return KAMSTA_OK;  // no room: stream the input instead
+  }
+  CU_TRY(ea);
   struct Free {
     kamsta_ctx* c;
     void* p;
     cudaStream_t s;
     ~Free() { ctx_free(c, p, s); }
   } fs{ctx_, smem, st_};
-  uint32_t* S = static_cast<uint32_t*>(smem);
+  uint64_t* scan_status = static_cast<uint64_t*>(smem);
+  uint32_t* S = reinterpret_cast<uint32_t*>(scan_status + scan_words);
   uint32_t* row_lo = S + cap_s;
-  uint32_t* fence = row_lo + cap_s;
+  uint32_t* row_hi = row_lo + cap_s;
+  uint32_t* pos = row_hi + cap_s;
+  uint32_t* fence = pos + cap_s;
   const int t0 = tick();
   CU_TRY(cudaMemsetAsync(ctx_->d_counters + kCMisc, 0, sizeof(DevCounters), st_));
   unsigned long long* cnt = &ctx_->d_counters[kCMisc].cnt[0];
-  k_outside_big<<<grid_for((n_ + 31) / 32), kBlock, 0, st_>>>(n_, big_, S, cap_s, cnt);
+  const uint32_t words = ceil_div(n_, 32);
+  const uint32_t gw = std::max<uint32_t>(
+      1, std::min<uint32_t>(ceil_div(words, kBlock), static_cast<uint32_t>(sms_) * 4));
+  const uint32_t chunk = ceil_div(words, gw);
+  k_outside_count<<<gw, kBlock, 0, st_>>>(n_, big_, chunk, cta_counts_, cnt);
+  k_fences<<<grid_for(nfence), kBlock, 0, st_>>>(in_, md_, fence);
   KS_TRY(fetch_counters());
   const uint64_t ns = ctx_->h_counters[kCMisc].cnt[0];
   if (ns > cap_s) return KAMSTA_OK;  // too many: stream the input instead
-  const int grid = grid_for(std::max<uint64_t>(ns * 32, 1));
-  // records are ordered by (min id << key_bits | max id); the batch's forest
-  // bitmap needs the src<dst copy's position in each record
+  const uint32_t nsu = static_cast<uint32_t>(ns);
+  // the records' order is that of their min ids; the batch's forest bitmap
+  // needs the src<dst copy's position in each record
   uint32_t key_bits = 1;
   while (key_bits < 32 && (1ull << key_bits) < n_) ++key_bits;
   const uint32_t canon = forest_bits_ != nullptr ? 1u : 0u;
-  // count (and find the rows), then write the surviving edges
-  k_fences<<<grid_for(nfence), kBlock, 0, st_>>>(in_, md_, fence);
-  k_row_scan<false><<<grid, kBlock, 0, st_>>>(in_, md_, n_, S, static_cast<uint32_t>(ns), row_lo,
-                                              fence, D_, big_, big_label_, wmin, wmax, canon,
-                                              key_bits,
-                                              nullptr, nullptr, 0,
-                                              &ctx_->d_counters[kCMisc].cnt[1], ctx_->d_err);
-  KS_TRY(fetch_counters());
-  const uint64_t k = ctx_->h_counters[kCMisc].cnt[1];
+  const int grid = grid_for(std::max<uint64_t>(ns * kRowLanes, 1));
+  uint64_t k = 0;
+  if (ns > 0) {
+    k_outside_write<<<gw, kBlock, 0, st_>>>(n_, big_, chunk, cta_counts_, S, cap_s);
+    k_row_find<<<grid_for(ns), kBlock, 0, st_>>>(in_, md_, fence, S, nsu, row_lo, row_hi);
+    k_row_scan<false><<<grid, kBlock, 0, st_>>>(in_, md_, n_, S, nsu, row_lo, row_hi, pos, fence,
+                                                D_, big_, big_label_, wmin, wmax, canon, nullptr,
+                                                nullptr, 0, ctx_->d_err);
+    // the last row's records, and the records before it
+    CU_TRY(cudaMemcpyAsync(&ctx_->h_samples[0], pos + ns - 1, sizeof(uint32_t),
+                           cudaMemcpyDeviceToHost, st_));
+    CU_TRY(exclusive_scan_u32(st_, pos, pos, ns, scan_status, &ctx_->d_counters[kCMisc].ticket,
+                              ctx_->d_err, sms_));
+    CU_TRY(cudaMemcpyAsync(&ctx_->h_samples[1], pos + ns - 1, sizeof(uint32_t),
+                           cudaMemcpyDeviceToHost, st_));
+    KS_TRY(fetch_counters());
+    k = uint64_t(ctx_->h_samples[0]) + ctx_->h_samples[1];
+  }
   KS_TRY(alloc_list(E, 1, std::max<uint64_t>(k, 1)));
   if (k > 0) {
     void* tmem = nullptr;
@@ -1236,15 +1261,13 @@ kamsta_status Solve::contract_rows(uint32_t wmin, uint32_t wmax, SegList* E, boo
     uint32_t* idx2 = reinterpret_cast<uint32_t*>(m + rb + 2 * kb + ib);
     uint32_t* counts = reinterpret_cast<uint32_t*>(m + rb + 2 * kb + 2 * ib);
     uint64_t* status = reinterpret_cast<uint64_t*>(m + rb + 2 * kb + 2 * ib + cb);
-    k_row_scan<true><<<grid, kBlock, 0, st_>>>(in_, md_, n_, S, static_cast<uint32_t>(ns), row_lo,
-                                               fence, D_, big_, big_label_, wmin, wmax, canon,
-                                               key_bits,
-                                               tmp, keys, k, &ctx_->d_counters[kCMisc].cnt[2],
-                                               ctx_->d_err);
+    k_row_scan<true><<<grid, kBlock, 0, st_>>>(in_, md_, n_, S, nsu, row_lo, row_hi, pos, fence,
+                                               D_, big_, big_label_, wmin, wmax, canon, tmp, keys,
+                                               k, ctx_->d_err);
     k_iota<<<grid_for(k), kBlock, 0, st_>>>(static_cast<uint32_t>(k), idx);
     int alt = 0;
     cudaError_t e = radix_sort_pairs_u32(st_, keys, keys2, idx, idx2, k,
-                                         static_cast<int>(2 * key_bits), counts, status,
+                                         static_cast<int>(key_bits), counts, status,
                                          &ctx_->d_counters[kCMisc].ticket, ctx_->d_err, &alt,
                                          sms_);
     if (e != cudaSuccess) return cuda_status(e, "radix sort (row scan)");

@@ -311,3 +311,31 @@ def test_long_rows_fold_their_minimum(kamsta, oracle, hub, lp):
         assert st["total_weight"] == w
         assert np.array_equal(oracle.canon_keys(f), oracle.canon_keys(ref))
     ctx.close()
+
+
+@pytest.mark.parametrize("rows", [(1, 8, 9), (255, 256, 257), (5000, 7, 33)])
+def test_row_scans_match_the_streamed_class(kamsta, oracle, rows):
+    """Outside rows around the lanes of a row (8) and the row a warp takes
+    whole (257 entries), last in the input and between other rows; a traced
+    solve contracts the heaviest class by row scans, the other one streams
+    it, and both write the same bytes."""
+    n0 = 100003
+    e0 = oracle.gen_gnm(n0, 1200000, 17)
+    rng = np.random.default_rng(5)
+    # every third id is left out of the graph; some of those become the rows
+    ids = np.arange(n0, dtype=np.uint32) * 3 // 2
+    und = [(int(ids[a]), int(ids[b]), int(w)) for a, b, w in e0[e0["src"] < e0["dst"]][::2].tolist()]
+    free = np.setdiff1d(np.arange(ids[-1]), ids)[[10, 2000, -10]]
+    for v, deg in zip(free, rows):
+        for u in rng.choice(ids, deg, replace=False):
+            und.append((min(int(v), int(u)), max(int(v), int(u)), 254 - int(rng.integers(0, 3))))
+    e, n = oracle.symmetric_from_undirected(und), int(ids[-1]) + 1
+    ctx = kamsta.Context(0)
+    got, k, st = _dev_solve(kamsta, ctx, e, n, kamsta.AlgorithmConfig(local_preprocessing=1))
+    want, kw, sw = _dev_solve(kamsta, ctx, e, n,
+                              kamsta.AlgorithmConfig(local_preprocessing=1, trace=True))
+    ref, w = oracle.kruskal(e, n)
+    assert st["row_scans"] == 0 and st["total_weight"] == sw["total_weight"] == w
+    assert k == kw == len(ref) and np.array_equal(got, want)
+    ctx.close()
+    assert sw["row_scans"] >= 1
