@@ -474,6 +474,7 @@ kamsta_status kamsta_ctx_create(int device, kamsta_ctx** out) {
       (e = cudaMallocHost(&c->h_counters, sizeof(DevCounters) * kCSlots)) != cudaSuccess ||
       (e = cudaMallocHost(&c->h_err, sizeof(uint32_t))) != cudaSuccess ||
       (e = cudaMallocHost(&c->h_samples, sizeof(uint32_t) * kSampleWords)) != cudaSuccess ||
+      (e = cudaMallocHost(&c->h_counts, sizeof(uint32_t) * kCountWords)) != cudaSuccess ||
       (e = cudaMallocHost(&c->h_state, kHostState)) != cudaSuccess ||
       (e = cudaEventCreate(&c->ev0)) != cudaSuccess ||
       (e = cudaEventCreate(&c->ev1)) != cudaSuccess) {
@@ -525,6 +526,7 @@ kamsta_status kamsta_ctx_destroy(kamsta_ctx* ctx) {
   if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
   if (ctx->h_err) cudaFreeHost(ctx->h_err);
   if (ctx->h_samples) cudaFreeHost(ctx->h_samples);
+  if (ctx->h_counts) cudaFreeHost(ctx->h_counts);
   if (ctx->h_state) cudaFreeHost(ctx->h_state);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);

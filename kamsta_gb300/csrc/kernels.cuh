@@ -1871,15 +1871,33 @@ __global__ void __launch_bounds__(kSampleBlock)
   if (threadIdx.x < 2) out[kSampleCount + threadIdx.x] = s_cnt[threadIdx.x];
 }
 
-// Same over a segmented list; prefix[s] = records in segments < s.
+// Same over a segmented list; the records before each segment are summed here,
+// one segment per thread.
+static_assert(kMaxSeg <= kSampleBlock, "one thread per segment");
 __global__ void __launch_bounds__(kSampleBlock)
-    k_sample_weights_seg(SegIn in, const uint64_t* __restrict__ prefix, uint64_t m,
-                         uint64_t seed, uint32_t* __restrict__ out) {
+    k_sample_weights_seg(SegIn in, uint64_t m, uint64_t seed, uint32_t* __restrict__ out) {
+  __shared__ uint64_t s_pre[kMaxSeg + 1];
+  __shared__ uint64_t s_warp[kSampleBlock / 32];
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  const uint64_t c = threadIdx.x < in.nseg ? in.count[threadIdx.x] : 0u;
+  uint64_t incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint64_t y = __shfl_up_sync(kFull, incl, o);
+    if (lane >= static_cast<uint32_t>(o)) incl += y;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  uint64_t before = 0;
+  for (uint32_t w = 0; w < warp; ++w) before += s_warp[w];
+  s_pre[threadIdx.x] = before + incl - c;
+  if (threadIdx.x == kSampleBlock - 1) s_pre[kMaxSeg] = before + incl;
+  __syncthreads();
   sample_sorted(
       [&](uint32_t i) {
         const uint64_t x = __umul64hi(mix64(seed + i), m);
-        const uint32_t sg = seg_find(prefix, in.nseg, x);
-        return in.base[static_cast<uint64_t>(sg) * in.cap + (x - prefix[sg])].w;
+        const uint32_t sg = seg_find(s_pre, in.nseg, x);
+        return in.base[static_cast<uint64_t>(sg) * in.cap + (x - s_pre[sg])].w;
       },
       out);
 }

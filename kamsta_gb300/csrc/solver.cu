@@ -234,6 +234,7 @@ static inline uint32_t ceil_div(uint64_t a, uint64_t b) {
   return static_cast<uint32_t>((a + b - 1) / b);
 }
 
+static_assert(kMaxOut * kMaxSeg == kCountWords, "the context holds one pass's counts");
 static_assert(kSampleCount == kSampleCap, "the context holds one sample");
 // Round passes over at most this many vertices use 4-record tiles.
 constexpr uint32_t kWideRoundN = 1u << 16;
@@ -357,7 +358,8 @@ class Solve {
   std::vector<uint32_t> plan_classes(bool as_preprocessed);
   kamsta_status sample_weights(const SegList* L, std::vector<uint32_t>* out);
   kamsta_status fetch_samples(std::vector<uint32_t>* out);
-  kamsta_status filter_rec(SegList* L, bool own, bool stop, int depth);
+  // last: no contraction follows this call's, so its labels are not needed
+  kamsta_status filter_rec(SegList* L, bool own, bool stop, int depth, bool last);
   kamsta_status run_boruvka();
   kamsta_status run_classes();
   // Plain rounds over the forest's edges alone; *done = false: not worth it,
@@ -466,7 +468,7 @@ class Solve {
   uint32_t *P_ = nullptr, *D_ = nullptr, *V_ = nullptr, *Vn_ = nullptr;
   uint32_t *dense_of_ = nullptr, *parent_ = nullptr, *msfoid_ = nullptr, *newid_ = nullptr;
   uint32_t *Rbuf_ = nullptr, *Obuf_ = nullptr, *msf_ = nullptr, *samples_ = nullptr;
-  uint64_t *minA_ = nullptr, *minB_ = nullptr, *prefix_ = nullptr;
+  uint64_t *minA_ = nullptr, *minB_ = nullptr;
   uint32_t* cta_counts_ = nullptr;  // per-CTA counts of the vertex scans
   uint32_t* big_ = nullptr;         // membership bitmap of the largest component
   void* coop_mem_ = nullptr;
@@ -504,7 +506,6 @@ kamsta_status Solve::alloc_fixed() {
   add(n + 64, 4);                             // Obuf
   add(n + 1, 8);
   add(n + 1, 8);  // minA minB
-  add(kMaxSeg + 1, 8);
   add(2 * kMaxSeg, 4);
   add(n / 32 + 2, 4);
   add(4, 8);  // dweight
@@ -523,7 +524,6 @@ kamsta_status Solve::alloc_fixed() {
   Obuf_ = A.take<uint32_t>(n + 64);
   minA_ = A.take<uint64_t>(n + 1);
   minB_ = A.take<uint64_t>(n + 1);
-  prefix_ = A.take<uint64_t>(kMaxSeg + 1);
   cta_counts_ = A.take<uint32_t>(2 * kMaxSeg);
   big_ = A.take<uint32_t>(n / 32 + 2);
   dweight_ = A.take<unsigned long long>(4);
@@ -783,7 +783,7 @@ kamsta_status Solve::pass(int phase, const SegList* src, const uint32_t* map, ui
       return KAMSTA_OK;
     }
     for (int c = 0; c < NOUT; ++c)
-      CU_TRY(cudaMemcpyAsync(outs[c]->h_count.data(), outs[c]->d_count, sizeof(uint32_t) * G,
+      CU_TRY(cudaMemcpyAsync(ctx_->h_counts + c * kMaxSeg, outs[c]->d_count, sizeof(uint32_t) * G,
                              cudaMemcpyDeviceToHost, st_));
     tolerate_overflow_ = true;
     const kamsta_status fs = fetch_counters();
@@ -792,6 +792,7 @@ kamsta_status Solve::pass(int phase, const SegList* src, const uint32_t* map, ui
     bool overflow = false;
     uint64_t kept = 0;
     for (int c = 0; c < NOUT; ++c) {
+      std::memcpy(outs[c]->h_count.data(), ctx_->h_counts + c * kMaxSeg, sizeof(uint32_t) * G);
       uint64_t sum = 0, mx = 0;
       for (uint32_t s = 0; s < G; ++s) {
         sum += outs[c]->h_count[s];
@@ -1096,11 +1097,7 @@ kamsta_status Solve::sample_weights(const SegList* L, std::vector<uint32_t>* out
   if (m == 0) return KAMSTA_OK;
   const int tp = tick();
   if (L) {
-    std::vector<uint64_t> pre(L->nseg + 1, 0);
-    for (uint32_t s = 0; s < L->nseg; ++s) pre[s + 1] = pre[s] + L->h_count[s];
-    CU_TRY(cudaMemcpyAsync(prefix_, pre.data(), sizeof(uint64_t) * (L->nseg + 1),
-                           cudaMemcpyHostToDevice, st_));
-    k_sample_weights_seg<<<1, kSampleBlock, 0, st_>>>(L->in(), prefix_, m, cfg_.seed, samples_);
+    k_sample_weights_seg<<<1, kSampleBlock, 0, st_>>>(L->in(), m, cfg_.seed, samples_);
   } else {
     k_sample_weights<<<1, kSampleBlock, 0, st_>>>(in_, m, n_, cfg_.seed, samples_);
   }
@@ -1555,8 +1552,12 @@ kamsta_status Solve::run_coop(bool* done) {
 
 kamsta_status Solve::coop_tail(SegList* L, bool own, bool prologue, Rounds* R, bool* ran,
                                bool* finalized) {
-  *ran = false;
-  coop_grid_ = coop_grid(L->total + R->nr, sms_);
+  *ran = *finalized = false;
+  const bool direct = direct_emit_ && R->r == 0;
+  *finalized = R->r == 0 && !final_contraction_ && n_ <= kCoopFinalizeN;
+  // (the label update is over all n vertices, however short the list: one CTA
+  // took 150 us for 2^20)
+  coop_grid_ = coop_grid(L->total + R->nr + (*finalized ? n_ / 4 : 0), sms_);
   const uint32_t nq = coop_grid_ * coop::kGroups;
   const kamsta_status s = [&]() -> kamsta_status {
     KS_TRY(coop_buffers((L->total + nq - 1) / nq, own ? L : nullptr));
@@ -1564,12 +1565,11 @@ kamsta_status Solve::coop_tail(SegList* L, bool own, bool prologue, Rounds* R, b
   }();
   if (s == KAMSTA_E_OOM) {
     coop_off_ = true;
+    *finalized = false;
     return KAMSTA_OK;
   }
   KS_TRY(s);
   *ran = true;
-  const bool direct = direct_emit_ && R->r == 0;
-  *finalized = R->r == 0 && !final_contraction_ && n_ <= kCoopFinalizeN;
   coop::Args a = coop_args(L);
   a.first = 1;
   a.nr0 = R->nr;
@@ -1774,7 +1774,7 @@ kamsta_status Solve::run_classes() {
 // (boruvka_recursive_setup, :173-225), recurse on what is left.  A light
 // share above 85% stops the next level (partition_edges,
 // filter_helpers.hpp:130-133).  L == nullptr is the directed input.
-kamsta_status Solve::filter_rec(SegList* L, bool own, bool stop, int depth) {
+kamsta_status Solve::filter_rec(SegList* L, bool own, bool stop, int depth, bool last) {
   const uint64_t m_und = L ? L->total : md_ / 2;  // the input holds m_directed/2 edges
   if (m_und == 0 || nreps_ <= 1) {
     if (own) free_list(L);
@@ -1783,7 +1783,10 @@ kamsta_status Solve::filter_rec(SegList* L, bool own, bool stop, int depth) {
   const double avg_degree = 2.0 * static_cast<double>(m_und) / static_cast<double>(n_);
   if (avg_degree <= static_cast<double>(cfg_.filter_threshold) || stop || 2 * m_und <= 1000 ||
       depth >= 48) {
-    KS_TRY(contract(L, 0, 0xffffffffu, 1.0));
+    final_contraction_ = last;
+    const kamsta_status cs = contract(L, 0, 0xffffffffu, 1.0);
+    final_contraction_ = false;
+    KS_TRY(cs);
     if (own) free_list(L);
     return KAMSTA_OK;
   }
@@ -1800,7 +1803,7 @@ kamsta_status Solve::filter_rec(SegList* L, bool own, bool stop, int depth) {
   if (own) free_list(L);
   const uint64_t tot = light->total + heavy->total;
   const bool stop_next = tot == 0 || static_cast<double>(light->total) / tot > 0.85;
-  KS_TRY(filter_rec(light, true, stop_next, depth + 1));
+  KS_TRY(filter_rec(light, true, stop_next, depth + 1, last && heavy->total == 0));
   if (nreps_ <= 1 || heavy->total == 0) {
     free_list(heavy);
     return KAMSTA_OK;
@@ -1810,10 +1813,10 @@ kamsta_status Solve::filter_rec(SegList* L, bool own, bool stop, int depth) {
   KS_TRY(pass<1>(KAMSTA_PHASE_CLASS_PASS, heavy, P_, 0, 0xffffffffu, nullptr, kouts, nullptr,
                  nullptr, 0, false));
   free_list(heavy);
-  return filter_rec(kept, true, false, depth + 1);
+  return filter_rec(kept, true, false, depth + 1, last);
 }
 
-kamsta_status Solve::run_filter_boruvka() { return filter_rec(nullptr, false, false, 0); }
+kamsta_status Solve::run_filter_boruvka() { return filter_rec(nullptr, false, false, 0, true); }
 
 // ---------------------------------------------------------------------------
 

@@ -75,6 +75,7 @@ enum CounterSlot : int { kCVertex = 0, kCEdge = 1, kCRep = 2, kCMisc = 3, kCSlot
 constexpr uint32_t kSampleCap = 4096;
 constexpr uint32_t kSampleWords = kSampleCap + 16;  // the sample, then its counters
 constexpr int kTimerEvents = 64;
+constexpr uint32_t kCountWords = 3 * 1024;  // segment counts of a pass's outputs
 constexpr size_t kHostState = 1024;  // bytes of kamsta_ctx::h_state
 constexpr int kInputPieces = 16;  // host input copied in this many pieces
 
@@ -104,6 +105,7 @@ struct kamsta_ctx {
   kamsta::DevCounters* h_counters = nullptr;  // pinned mirror
   uint32_t* h_err = nullptr;
   uint32_t* h_samples = nullptr;  // pinned: the sorted samples
+  uint32_t* h_counts = nullptr;   // pinned: a pass's segment counts
   void* h_state = nullptr;        // pinned: head of the cooperative solve's state
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t tev[kamsta::kTimerEvents] = {};  // per-phase timing events
