@@ -20,16 +20,13 @@
 
 #include "../../include/kamsta_gpu.h"
 #include "common.cuh"
-#include "small_solve.cuh"
+#include "small_found.cuh"
 
 namespace kamsta {
 namespace noalloc {
 
 constexpr uint32_t kMaxN = small::kMaxN;
 constexpr uint64_t kMaxMd = small::kMaxMd;
-// Small graphs take a smaller CTA: their phases are as short as its barriers.
-constexpr int kThreads = 1024, kThreadsFew = 256;
-constexpr uint64_t kFewMd = 1ull << 14;
 constexpr size_t kScratchBytes = small::kScratchBytes;
 using NaResult = small::Result;
 
@@ -41,7 +38,7 @@ using NaResult = small::Result;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kamsta::noalloc::kScratchBytes];
 
 namespace kamsta {
-namespace noalloc {
+namespace small {
 
 // The whole solve in one CTA (small_solve.cuh), forest edges in the order
 // the rounds find them; the result header sits at the start of the scratch.
@@ -50,13 +47,36 @@ namespace noalloc {
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 1)
     k_noalloc_boruvka(const uint32_t* __restrict__ in, uint32_t md, uint32_t n,
-                      unsigned char* __restrict__ scratch, uint32_t* __restrict__ out) {
+                      unsigned char* __restrict__ scratch, uint32_t* __restrict__ out,
+                      uint32_t check_order) {
   extern __shared__ __align__(16) unsigned char s_raw[];
-  small::solve<THREADS, small::Out::kFound, small::Size::kFull>(
-      in, md, n, scratch, out, reinterpret_cast<NaResult*>(scratch), s_raw, true);
+  solve<THREADS, Out::kFound, Size::kFull>(in, md, n, scratch, out,
+                                           reinterpret_cast<Result*>(scratch), s_raw, true,
+                                           check_order != 0);
 }
 
-}  // namespace noalloc
+cudaError_t found_setup() {
+  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  const int smem = static_cast<int>(kSharedFull);
+  cudaError_t e = cudaFuncSetAttribute(k_noalloc_boruvka<kFoundThreads>, attr, smem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_noalloc_boruvka<kFoundThreadsFew>, attr, smem);
+  return e;
+}
+
+cudaError_t found_launch(const uint32_t* in, uint32_t md, uint32_t n, unsigned char* scratch,
+                         uint32_t* out, bool check_order, cudaStream_t st) {
+  const size_t smem = shared_bytes(n);
+  const uint32_t check = check_order ? 1u : 0u;
+  if (md <= kFoundFewMd)
+    k_noalloc_boruvka<kFoundThreadsFew>
+        <<<1, kFoundThreadsFew, smem, st>>>(in, md, n, scratch, out, check);
+  else
+    k_noalloc_boruvka<kFoundThreads>
+        <<<1, kFoundThreads, smem, st>>>(in, md, n, scratch, out, check);
+  return cudaGetLastError();
+}
+
+}  // namespace small
 }  // namespace kamsta
 
 namespace kamsta {
@@ -87,11 +107,7 @@ kamsta_status scratch_for_current_device(unsigned char** out) {
     void* p = nullptr;
     e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
     if (e != cudaSuccess) return kamsta::cuda_status(e, "cudaGetSymbolAddress(scratch)");
-    using namespace kamsta::noalloc;
-    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    const int smem = static_cast<int>(kamsta::small::kSharedFull);
-    e = cudaFuncSetAttribute(k_noalloc_boruvka<kThreads>, attr, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_noalloc_boruvka<kThreadsFew>, attr, smem);
+    e = kamsta::small::found_setup();
     if (e != cudaSuccess) return kamsta::cuda_status(e, "cudaFuncSetAttribute(k_noalloc_boruvka)");
     g_scratch_ptr[dev] = p;
   }
@@ -123,13 +139,9 @@ extern "C" kamsta_status kamsta_mst_boruvka_noalloc(const kamsta_wedge* d_edges,
   kamsta_status s = scratch_for_current_device(&scratch);
   if (s != KAMSTA_OK) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const uint32_t* in = reinterpret_cast<const uint32_t*>(d_edges);
-  uint32_t* out = reinterpret_cast<uint32_t*>(d_out);
-  const uint32_t md = static_cast<uint32_t>(m_directed);
-  const size_t smem = kamsta::small::shared_bytes(n);
-  if (md <= kFewMd) k_noalloc_boruvka<kThreadsFew><<<1, kThreadsFew, smem, st>>>(in, md, n, scratch, out);
-  else k_noalloc_boruvka<kThreads><<<1, kThreads, smem, st>>>(in, md, n, scratch, out);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = kamsta::small::found_launch(
+      reinterpret_cast<const uint32_t*>(d_edges), static_cast<uint32_t>(m_directed), n, scratch,
+      reinterpret_cast<uint32_t*>(d_out), false, st);
   if (e != cudaSuccess) return kamsta::cuda_status(e, "k_noalloc_boruvka launch");
   NaResult h{};
   e = cudaMemcpyAsync(&h, scratch, sizeof(h), cudaMemcpyDeviceToHost, st);

@@ -25,6 +25,7 @@
 
 #include "kernels.cuh"
 #include "rounds_coop.cuh"
+#include "small_found.cuh"
 #include "solver.cuh"
 #include "sort_gen.cuh"
 
@@ -253,6 +254,11 @@ constexpr uint32_t kTailN = 1u << 23;
 // the update's gathers need the full occupancy of its own kernels.
 constexpr uint32_t kCoopFinalizeN = 1u << 22;
 
+// Plain rounds of at most this many entries (and 2^15 vertices) are solved by
+// one CTA: a few phases of a microsecond or two against the cooperative
+// grid's barriers and launches.  Grid / one CTA, us per call: 4100 entries 105
+// / 66, 8200 120 / 74, 32800 121 / 104, 65500 133 / 154.
+constexpr uint64_t kOneCtaMd = 1ull << 15;
 // Plain rounds are replayed on the forest (run_sparse) for inputs of at least
 // kSparseMinMd entries with 24 or more entries per vertex, and from
 // kSparseFarMd entries on with 14 or more when most edges join far ids.
@@ -362,6 +368,9 @@ class Solve {
   kamsta_status filter_rec(SegList* L, bool own, bool stop, int depth, bool last);
   kamsta_status run_boruvka();
   kamsta_status run_classes();
+  // Plain rounds of a small graph in one CTA; *done = false: no memory for its
+  // scratch, or a device check that the other rounds report.
+  kamsta_status run_one_cta(bool* done);
   // Plain rounds over the forest's edges alone; *done = false: not worth it,
   // or no memory for it.
   kamsta_status run_sparse(bool* done);
@@ -401,7 +410,8 @@ class Solve {
   uint64_t coop_cap_ = 0;     // records per segment of the two buffers
   Rec* coop_buf_[2] = {nullptr, nullptr};
   SegList* coop_list_[2] = {nullptr, nullptr};  // what holds them
-  bool coop_done_ = false;    // the solve's forest is written
+  bool coop_done_ = false;    // the solve's forest is written, its weight known
+  uint64_t weight_ = 0;
   kamsta_status run_filter_boruvka();
   // ---- debugging (KAMSTA_DEBUG_CHECKS=1): host-side invariant checks
   kamsta_status debug_list(const char* where, const SegList& L, uint64_t nlabels);
@@ -1545,6 +1555,7 @@ kamsta_status Solve::run_coop(bool* done) {
   // per record: read, two labels, written again, two minima; per vertex of a
   // round: minimum, record, partner, parent, label and compaction
   account(KAMSTA_PHASE_ROUND_EDGES, h.sum_m * 56 + h.sum_n * 60, coop_launches_);
+  weight_ = h.weight;
   coop_done_ = true;
   *done = true;
   return KAMSTA_OK;
@@ -1717,6 +1728,52 @@ kamsta_status Solve::run_sparse(bool* done) {
   const kamsta_status r = rounds(E, true);
   direct_emit_ = final_contraction_ = false;
   KS_TRY(r);
+  *done = true;
+  return KAMSTA_OK;
+}
+
+kamsta_status Solve::run_one_cta(bool* done) {
+  *done = false;
+  void* mem = nullptr;
+  if (ctx_alloc(ctx_, &mem, small::kScratchBytes, st_) != cudaSuccess) {
+    cudaGetLastError();
+    return KAMSTA_OK;
+  }
+  struct Free {
+    kamsta_ctx* c;
+    void* p;
+    cudaStream_t s;
+    ~Free() { ctx_free(c, p, s); }
+  } fm{ctx_, mem, st_};
+  if (io_) KS_TRY(wait_input(io_->pieces - 1));
+  input_complete_ = true;
+  if (!ctx_->found_ready) {
+    CU_TRY(small::found_setup());
+    ctx_->found_ready = true;
+  }
+  const bool validate = (cfg_.flags & KAMSTA_FLAG_VALIDATE) != 0;
+  const int t0 = tick();
+  CU_TRY(small::found_launch(in_, static_cast<uint32_t>(md_), n_,
+                             static_cast<unsigned char*>(mem),
+                             reinterpret_cast<uint32_t*>(d_out_), validate, st_));
+  tock(KAMSTA_PHASE_ROUND_EDGES, t0);
+  static_assert(sizeof(small::Result) <= kHostState, "pinned mirror of the result");
+  CU_TRY(cudaMemcpyAsync(ctx_->h_state, mem, sizeof(small::Result), cudaMemcpyDeviceToHost, st_));
+  CU_TRY(cudaStreamSynchronize(st_));
+  resolve();
+  const small::Result& r = *static_cast<const small::Result*>(ctx_->h_state);
+  // ids beyond n are only an error when the input is to be validated
+  if (r.err & (validate ? ~0u : ~static_cast<uint32_t>(kErrRange))) {
+    *ctx_->h_err = r.err;
+    const kamsta_status s = check_err();
+    return s == KAMSTA_E_INPUT ? s : KAMSTA_OK;
+  }
+  msf_count_ = r.count;
+  weight_ = r.weight;
+  rounds_ += r.rounds;
+  levels_ += 1;
+  account(KAMSTA_PHASE_ROUND_EDGES, md_ * 12 + r.count * 24, 1);
+  coop_done_ = true;
   *done = true;
   return KAMSTA_OK;
 }
@@ -1906,15 +1963,21 @@ kamsta_status Solve::run(Algo algo, kamsta_wedge* d_out, SolveOut* out) {
     std::vector<uint32_t> thr_desc = plan_classes(classes);
     bounds_.assign(thr_desc.rbegin(), thr_desc.rend());
   }
-  k_init_vertices<<<grid_for(n_), kBlock, 0, st_>>>(n_, minA_, P_, V_, D_);
-  account(KAMSTA_PHASE_FINALIZE, uint64_t(n_) * 20, 1);
   nreps_ = n_;
   msf_count_ = 0;
   d_out_ = d_out;
   direct_count_ = 0;
-  CU_TRY(cudaMemsetAsync(dweight_, 0, sizeof(unsigned long long), st_));
-  CU_TRY(cudaMemsetAsync(ctx_->d_err, 0, sizeof(uint32_t), st_));
-  KS_TRY(algo == Algo::kBoruvka ? run_boruvka() : run_filter_boruvka());
+  bool done = false;
+  if (algo == Algo::kBoruvka && bounds_.empty() && forest_bits_ == nullptr && coop_options() &&
+      n_ <= small::kMaxN && md_ <= kOneCtaMd)
+    KS_TRY(run_one_cta(&done));
+  if (!done) {
+    k_init_vertices<<<grid_for(n_), kBlock, 0, st_>>>(n_, minA_, P_, V_, D_);
+    account(KAMSTA_PHASE_FINALIZE, uint64_t(n_) * 20, 1);
+    CU_TRY(cudaMemsetAsync(dweight_, 0, sizeof(unsigned long long), st_));
+    CU_TRY(cudaMemsetAsync(ctx_->d_err, 0, sizeof(uint32_t), st_));
+    KS_TRY(algo == Algo::kBoruvka ? run_boruvka() : run_filter_boruvka());
+  }
   // forest output (written by the cooperative rounds themselves)
   if (!coop_done_) CU_TRY(cudaMemsetAsync(ctx_->d_counters + kCMisc, 0, sizeof(DevCounters), st_));
   if (coop_done_) {
@@ -1937,7 +2000,7 @@ kamsta_status Solve::run(Algo algo, kamsta_wedge* d_out, SolveOut* out) {
   CU_TRY(cudaEventRecord(ctx_->ev1, st_));
   out->count = msf_count_;
   if (coop_done_) {
-    out->weight = static_cast<const coop::State*>(ctx_->h_state)->weight;
+    out->weight = weight_;
     if (stats_) CU_TRY(cudaEventSynchronize(ctx_->ev1));
   } else {
     KS_TRY(fetch_counters());

@@ -93,6 +93,7 @@ struct kamsta_ctx {
   // CTAs per SM of the small-graph kernels: tiny, compact by CTA size (256,
   // 512, 1024), full; 0 = not asked yet
   int small_per_sm[5] = {};
+  bool found_ready = false;  // small::found_setup has run
   // single-graph tiles (kamsta_autotune_tiles); 0 = built-in default
   uint32_t tune_dir_items = 0;      // entries per thread of the first pass
   uint32_t tune_seg_items = 0;      // records per thread of the list passes
