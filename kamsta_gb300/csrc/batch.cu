@@ -9,7 +9,9 @@
 // of thousands of tiny ones), and the forest is then split back per graph:
 //   k_batch_gather   copy the wave's inputs into one union array, adding
 //                    voff to src/dst (u32 words, coalesced); an id >= n_g is
-//                    replaced by an id the solver skips and flags graph g
+//                    replaced by an id the solver skips and flags graph g.
+//                    Large unions of aligned graphs skip the copy: the
+//                    solver's passes read them in place (union_in_place)
 //   k_batch_order    (KAMSTA_FLAG_VALIDATE) per-graph (src,dst) order check
 //   solve_device     the single-graph solver over the union; the forest comes
 //                    back as one bit per union entry (its src<dst copy)
@@ -250,6 +252,7 @@ __global__ void k_batch_bounds(WaveTable t, const uint32_t* __restrict__ bits,
 // position is searched once per block step; a thread walks on from it (the
 // union's graphs are larger than a step's 8192 positions, so a step crosses
 // at most a boundary or two).
+// A null `uni` reads the graphs in place (their ids are not shifted).
 __global__ void __launch_bounds__(kBatchBlock)
     k_batch_scatter(WaveTable t, const uint32_t* __restrict__ uni,
                     const uint32_t* __restrict__ bits, const uint32_t* __restrict__ pre,
@@ -276,6 +279,7 @@ __global__ void __launch_bounds__(kBatchBlock)
         constexpr int kB = 4;
         uint64_t ps[kB];
         uint32_t e0[kB], e1[kB], e2[kB];
+        uint32_t gl = g;
         int c = 0;
 #pragma unroll
         for (int k = 0; k < kB; ++k) {
@@ -287,7 +291,9 @@ __global__ void __launch_bounds__(kBatchBlock)
 #pragma unroll
         for (int k = 0; k < kB; ++k) {
           if (k >= c) break;
-          const uint32_t* e = uni + 3 * ps[k];
+          if (!uni)
+            while (ps[k] >= t.eoff[gl + 1]) ++gl;
+          const uint32_t* e = uni ? uni + 3 * ps[k] : t.edges[gl] + 3 * (ps[k] - t.eoff[gl]);
           e0[k] = e[0];
           e1[k] = e[1];
           e2[k] = e[2];
@@ -296,7 +302,7 @@ __global__ void __launch_bounds__(kBatchBlock)
         for (int k = 0; k < kB; ++k) {
           if (k >= c) break;
           while (ps[k] >= t.eoff[g + 1]) ++g;
-          const uint32_t v = static_cast<uint32_t>(t.voff[g]);
+          const uint32_t v = uni ? static_cast<uint32_t>(t.voff[g]) : 0u;
           const uint32_t wt = e2[k];
           uint32_t* o = t.out[g] + 3 * (rank - t.begin[g]);
           o[0] = e0[k] - v;
@@ -601,6 +607,35 @@ kamsta_status launch_small(kamsta_ctx* ctx, kamsta_graph_desc* g, const std::vec
   return KAMSTA_OK;
 }
 
+// Whether the union of g[0..G) is read in place: large enough, every graph
+// aligned for the bulk copies and larger than a tile of the pass, no graph
+// with half of the vertices (its heaviest edges go row by row, from an array),
+// and no output over an input (inputs are read until the forest is written).
+bool union_in_place(const kamsta_graph_desc* g, uint32_t G, const kamsta_cfg& cfg, uint64_t M,
+                    uint64_t N) {
+  if ((cfg.flags & KAMSTA_FLAG_VALIDATE) || M < kUnionMinMd || M + 3ull * G >= (1ull << 32))
+    return false;
+  for (uint32_t i = 0; i < G; ++i)
+    if ((reinterpret_cast<uintptr_t>(g[i].edges) & 15u) || g[i].m_directed < kUnionMinGraph ||
+        2ull * g[i].n > N)
+      return false;
+  std::vector<std::pair<uintptr_t, uintptr_t>> in(G);  // (start, end), by start
+  for (uint32_t i = 0; i < G; ++i) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(g[i].edges);
+    in[i] = {a, a + g[i].m_directed * sizeof(kamsta_wedge)};
+  }
+  std::sort(in.begin(), in.end());
+  for (uint32_t i = 1; i < G; ++i) in[i].second = std::max(in[i].second, in[i - 1].second);
+  for (uint32_t i = 0; i < G; ++i) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(g[i].out);
+    // the inputs that start before the output's end
+    const auto it = std::lower_bound(
+        in.begin(), in.end(), std::make_pair(a + g[i].n * sizeof(kamsta_wedge), uintptr_t(0)));
+    if (it != in.begin() && std::prev(it)->second > a) return false;
+  }
+  return true;
+}
+
 // The union path for the graphs g[0..G).
 kamsta_status solve_union(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint32_t G,
                           const kamsta_cfg& cfg, bool host_buffers, cudaStream_t st,
@@ -611,12 +646,16 @@ kamsta_status solve_union(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint
     eoff[i + 1] = eoff[i] + g[i].m_directed;
     voff[i + 1] = voff[i] + g[i].n;
   }
-  const uint64_t M = eoff[G], N = voff[G];
+  const uint64_t N = voff[G];
   if (N >= kBatchMaxVertices) {
     set_error("batch: a wave holds too many vertices");
     return KAMSTA_E_INPUT;
   }
-  ws->entries = M;
+  ws->entries = eoff[G];
+  const bool in_place = !host_buffers && union_in_place(g, G, cfg, eoff[G], N);
+  if (in_place)  // every graph starts on a 16-byte boundary
+    for (uint32_t i = 0; i < G; ++i) eoff[i + 1] = (eoff[i] + g[i].m_directed + 3) & ~3ull;
+  const uint64_t M = eoff[G];
   ws->vertices = N;
   // table layout in one device block
   const size_t o_edges = 0;
@@ -627,11 +666,12 @@ kamsta_status solve_union(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint
   const size_t o_begin = o_n + up256(sizeof(uint32_t) * G);
   const size_t o_weight = o_begin + up256(sizeof(uint64_t) * (G + 1));
   const size_t o_err = o_weight + up256(sizeof(uint64_t) * G);
-  const size_t tbytes = o_err + up256(sizeof(uint32_t) * G);
+  const size_t o_graphs = o_err + up256(sizeof(uint32_t) * G);
+  const size_t tbytes = o_graphs + (in_place ? up256(sizeof(UnionGraph) * G) : 0);
   std::vector<unsigned char> h(tbytes, 0);
   PoolBuf tbuf, ubuf, obuf;
   B_TRY(tbuf.alloc(ctx, tbytes, st));
-  B_TRY(ubuf.alloc(ctx, std::max<uint64_t>(M, 1) * sizeof(kamsta_wedge), st));
+  if (!in_place) B_TRY(ubuf.alloc(ctx, std::max<uint64_t>(M, 1) * sizeof(kamsta_wedge), st));
   kamsta_wedge* uni = static_cast<kamsta_wedge*>(ubuf.p);
   unsigned char* d = static_cast<unsigned char*>(tbuf.p);
   // host buffers: outputs are staged in one device buffer, graph g at the
@@ -654,6 +694,10 @@ kamsta_status solve_union(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint
         ho[i] = reinterpret_cast<uint32_t*>(g[i].out);
       }
       reinterpret_cast<uint32_t*>(h.data() + o_n)[i] = g[i].n;
+      if (in_place)
+        reinterpret_cast<UnionGraph*>(h.data() + o_graphs)[i] =
+            UnionGraph{he[i], eoff[i], static_cast<uint32_t>(g[i].m_directed), g[i].n,
+                       static_cast<uint32_t>(voff[i]), 0};
     }
     std::memcpy(h.data() + o_eoff, eoff.data(), sizeof(uint64_t) * (G + 1));
     std::memcpy(h.data() + o_voff, voff.data(), sizeof(uint64_t) * (G + 1));
@@ -685,7 +729,7 @@ kamsta_status solve_union(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint
       ++launches;
     }
   }
-  if (M) {
+  if (M && !in_place) {
     const uint64_t words = 3 * M;
     const uint64_t chunk = static_cast<uint64_t>(kBatchBlock) * kGatherWords;
     const uint64_t blocks = std::min<uint64_t>((words + chunk - 1) / chunk, sms * 16ull);
@@ -705,8 +749,9 @@ kamsta_status solve_union(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint
   B_TRY(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * (W + 1), st));
   SolveOut so;
   kamsta_stats sst;
+  const UnionIn uin{reinterpret_cast<const UnionGraph*>(d + o_graphs), G, t.err};
   B_KTRY(solve_device(ctx, algo, uni, M, static_cast<uint32_t>(N), ucfg, nullptr, &so, &sst, st,
-                      bits));
+                      bits, nullptr, in_place ? &uin : nullptr));
   launches += sst.gpu_launches;
   ws->solve_ms = sst.device_ms;
   // ---- split: ranks of the set bits (word popcounts + exclusive scan), the
@@ -735,7 +780,7 @@ kamsta_status solve_union(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint
   }
   B_TRY(cudaGetLastError());
   // ---- per-graph results back to the host descriptors
-  std::vector<unsigned char> back(tbytes - o_begin);
+  std::vector<unsigned char> back(o_graphs - o_begin);
   B_TRY(cudaMemcpyAsync(back.data(), d + o_begin, back.size(), cudaMemcpyDeviceToHost, st));
   uint32_t derr = 0;
   B_TRY(cudaMemcpyAsync(ctx->h_err, ctx->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));

@@ -331,4 +331,17 @@ __device__ __forceinline__ void tile_rank(const uint8_t (&cls)[ITEMS],
     if (cls[j] != 0xff) offs[j] += smem[cls[j] * ROWS + j * WARPS + warp];
 }
 
+// A graph of a union that is read in place (batches): its entries are the
+// union's entries [eoff, eoff + md) -- eoff a multiple of 4, up to 3 unused
+// entries before the next graph -- and its vertices the union's [voff, voff +
+// n).  Every graph holds at least kUnionMinGraph entries, more than a tile of
+// the pass that reads it.
+struct UnionGraph {
+  const uint32_t* edges;  // 16-byte aligned
+  uint64_t eoff;
+  uint32_t md, n, voff;
+  uint32_t pad;
+};
+constexpr uint64_t kUnionMinGraph = 3072;
+
 }  // namespace kamsta

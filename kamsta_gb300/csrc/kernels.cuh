@@ -82,6 +82,9 @@ struct PassArgs {
   uint32_t validate;  // check id range and (src,dst) order (directed source)
   uint32_t aligned16; // directed source base is 16-byte aligned
   uint32_t cta_base;  // segment / chunk index of block 0 (a pass launched in groups)
+  const UnionGraph* ug;  // directed source read in place: its graphs,
+  uint32_t ng;           // their number,
+  uint32_t* gerr;        // and per graph whether an id was out of range
   // List passes of late rounds, whose next round has few labels: the
   // minimum of labels [0, smin_n) is taken per CTA in shared memory and
   // flushed with one reduction per label at the end (0 = off).  With few
@@ -325,7 +328,14 @@ constexpr size_t kDirDynSmem = dir_dyn_smem(kItemsDir);
 // queue up on the row's one word.  R-MAT 2^22, degree 16: 342 -> 240 us.  A
 // variant of its own, for inputs whose sample finds long rows: the test alone
 // cost G(n,m) 2^26/2^30 0.2 to 0.7 of 6.1 ms.
-template <int NOUT, int ITEMS = kItemsDir, bool MAPPED = false, bool HUB = false>
+//
+// UNION: the source is a union of graphs read in place.  A tile lies in one
+// graph or two; thread 0, which copies its runs, leaves them in shared memory,
+// and each item takes its graph's vertex offset from there.  (A union copied
+// together first costs a pass of 24 bytes per entry, 1.85 ms for 192 graphs
+// of 2^8..2^20 vertices; the batch took 11.96 ms with it, 10.81 in place.)
+template <int NOUT, int ITEMS = kItemsDir, bool MAPPED = false, bool HUB = false,
+          bool UNION = false>
 __global__ void __launch_bounds__(kBlock, ITEMS <= 8 ? 4 : 3)
     k_pass_dir(const uint32_t* __restrict__ in, PassArgs p) {
   constexpr uint32_t kDirTile = dir_tile(ITEMS);
@@ -350,11 +360,64 @@ __global__ void __launch_bounds__(kBlock, ITEMS <= 8 ? 4 : 3)
       bulk_load(s_words + stage * kDirStageWords,
                 in + (lo + static_cast<uint64_t>(k) * kDirTile) * 3, bytes16, &s_bar[stage]);
   };
+  // UNION: the runs of each stage's tile (t0, t1: its items; loose: the first
+  // word the bulk copy left out)
+  struct Run {
+    const uint32_t* src;
+    uint32_t t0, t1, loose, voff, n, g;
+  };
+  __shared__ Run s_run[UNION ? 2 : 1][2];
+  uint32_t gi = 0;  // thread 0: graph of the next tile's first entry
+  auto issue_union = [&](uint32_t k, int stage) {  // thread 0 only
+    const uint64_t b = lo + static_cast<uint64_t>(k) * kDirTile, e = b + tile_items(k);
+    uint32_t bytes = 0;
+    for (int r = 0; r < 2; ++r) {
+      Run& q = s_run[UNION ? stage : 0][r];
+      q = Run{nullptr, 0, 0, 0, 0, 0, 0};
+      // the first graph that ends behind b, then the one after it
+      if (r == 0)
+        while (gi + 1 < p.ng && p.ug[gi].eoff + p.ug[gi].md <= b) ++gi;
+      const uint32_t g = gi + r;
+      if (g >= p.ng) continue;
+      const UnionGraph u = p.ug[g];
+      const uint64_t x = u.eoff > b ? u.eoff : b, y = u.eoff + u.md < e ? u.eoff + u.md : e;
+      if (x >= y) continue;
+      q.src = u.edges + (x - u.eoff) * 3;
+      q.t0 = static_cast<uint32_t>(x - b);
+      q.t1 = static_cast<uint32_t>(y - b);
+      const uint32_t part = ((q.t1 - q.t0) * 12u) & ~15u;
+      q.loose = q.t0 * 3 + part / 4;
+      q.voff = u.voff;
+      q.n = u.n;
+      q.g = g;
+      bytes += part;
+    }
+    fence_proxy_async_smem();
+    mbar_arrive_expect_tx(&s_bar[stage], bytes);
+    for (int r = 0; r < 2; ++r) {
+      const Run& q = s_run[UNION ? stage : 0][r];
+      const uint32_t part = (q.loose - q.t0 * 3) * 4;
+      if (part)
+        bulk_load(s_words + stage * kDirStageWords + q.t0 * 3, q.src, part, &s_bar[stage]);
+    }
+  };
   if (threadIdx.x == 0) {
     mbar_init(&s_bar[0], 1);
     mbar_init(&s_bar[1], 1);
     fence_mbar_init();
-    if (tma && ntile > 0) issue(0, 0);
+    if constexpr (UNION) {
+      if (ntile > 0) {
+        uint32_t l = 0, h = p.ng;  // the last graph that starts at or before lo
+        while (h - l > 1) {
+          const uint32_t mid = (l + h) >> 1;
+          if (p.ug[mid].eoff <= lo) l = mid; else h = mid;
+        }
+        gi = l;
+        issue_union(0, 0);
+      }
+    } else {
+      if (tma && ntile > 0) issue(0, 0);
+    }
   }
   __syncthreads();
   uint64_t run[NOUT];
@@ -367,7 +430,25 @@ __global__ void __launch_bounds__(kBlock, ITEMS <= 8 ? 4 : 3)
     const uint64_t base = lo + static_cast<uint64_t>(k) * kDirTile;
     const uint32_t cnt = tile_items(k);
     uint32_t first_plain = 0;
-    if (tma) {
+    Run r0, r1;
+    if constexpr (UNION) {
+      if (threadIdx.x == 0) s_ok = mbar_wait(&s_bar[stage], (k >> 1) & 1u, p.err) ? 1u : 0u;
+      __syncthreads();  // also: every thread is done with tile k-1 and its stage
+      if (!s_ok) return;
+      r0 = s_run[UNION ? stage : 0][0];
+      r1 = s_run[UNION ? stage : 0][1];
+      if (threadIdx.x == 0 && k + 1 < ntile) issue_union(k + 1, stage ^ 1);
+      // the last words of graphs that end in this tile
+      const bool ends = r0.loose < 3 * r0.t1 || r1.loose < 3 * r1.t1;  // (the same in all threads)
+      if (ends) {
+        for (uint32_t i = r0.loose + threadIdx.x; i < 3 * r0.t1; i += kBlock)
+          words[i] = r0.src[i - 3 * r0.t0];
+        for (uint32_t i = r1.loose + threadIdx.x; i < 3 * r1.t1; i += kBlock)
+          words[i] = r1.src[i - 3 * r1.t0];
+        __syncthreads();
+      }
+      first_plain = 3 * cnt;
+    } else if (tma) {
       if (threadIdx.x == 0) s_ok = mbar_wait(&s_bar[stage], (k >> 1) & 1u, p.err) ? 1u : 0u;
       __syncthreads();  // also: every thread is done with tile k-1 and its stage
       if (!s_ok) return;
@@ -403,7 +484,50 @@ __global__ void __launch_bounds__(kBlock, ITEMS <= 8 ? 4 : 3)
       }
     }
     uint8_t cls[kItemsDir];
-    if constexpr (!MAPPED) {  // original ids: no label reads
+    if constexpr (UNION) {
+      uint32_t ss[kItemsDir], dd[kItemsDir], ww[kItemsDir];
+      bool keep[kItemsDir];
+#pragma unroll
+      for (int j = 0; j < kItemsDir; ++j) {
+        const uint32_t t = j * kBlock + threadIdx.x;
+        const bool second = t >= r1.t0 && t < r1.t1;
+        const uint32_t lim = second ? r1.n : r0.n, voff = second ? r1.voff : r0.voff;
+        const bool in_graph = second || (t >= r0.t0 && t < r0.t1);
+        ss[j] = words[3 * t];
+        dd[j] = words[3 * t + 1];
+        ww[j] = words[3 * t + 2];
+        keep[j] = false;
+        if (!in_graph) continue;
+        if (ss[j] >= lim || dd[j] >= lim) {
+          atomicOr(&p.gerr[second ? r1.g : r0.g], 1u);
+          continue;
+        }
+        if (!(ss[j] < dd[j]) || ww[j] < p.wmin || ww[j] > p.wmax) continue;
+        ss[j] += voff;
+        dd[j] += voff;
+        ++cand;
+        keep[j] = true;
+      }
+      uint32_t la[kItemsDir], lb[kItemsDir];
+      if constexpr (MAPPED) {
+        relabel_batch<kItemsDir>(p, ss, dd, keep, la, lb);
+      } else {
+#pragma unroll
+        for (int j = 0; j < kItemsDir; ++j) {
+          la[j] = ss[j];
+          lb[j] = dd[j];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kItemsDir; ++j) {
+        cls[j] = 0xff;
+        if (!keep[j]) continue;
+        const uint32_t t = j * kBlock + threadIdx.x;
+        words[3 * t] = la[j];  // item t belongs to this thread alone
+        words[3 * t + 1] = lb[j];
+        cls[j] = weight_class<NOUT>(ww[j], p);
+      }
+    } else if constexpr (!MAPPED) {  // original ids: no label reads
       const bool hub = HUB && p.min_partner && words[0] == words[3 * (cnt - 1)];
       if (hub) {
         const uint32_t row = words[0];
@@ -1869,6 +1993,25 @@ __global__ void __launch_bounds__(kSampleBlock)
   }
   __syncthreads();
   if (threadIdx.x < 2) out[kSampleCount + threadIdx.x] = s_cnt[threadIdx.x];
+}
+
+// Same over a union read in place (an unused entry counts as its graph's last).
+__global__ void __launch_bounds__(kSampleBlock)
+    k_sample_weights_union(const UnionGraph* __restrict__ ug, uint32_t ng, uint64_t m,
+                           uint64_t seed, uint32_t* __restrict__ out) {
+  sample_sorted(
+      [&](uint32_t i) {
+        const uint64_t pos = __umul64hi(mix64(seed + i), m);
+        uint32_t lo = 0, hi = ng;  // the last graph that starts at or before pos
+        while (hi - lo > 1) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (ug[mid].eoff <= pos) lo = mid; else hi = mid;
+        }
+        const uint64_t x = pos - ug[lo].eoff, last = ug[lo].md - 1u;
+        return ug[lo].edges[3 * (x < last ? x : last) + 2];
+      },
+      out);
+  if (threadIdx.x < 2) out[kSampleCount + threadIdx.x] = 0;
 }
 
 // Same over a segmented list; the records before each segment are summed here,

@@ -313,6 +313,7 @@ class Solve {
   uint32_t* forest_bits_ = nullptr;
   // host input arriving in pieces / early forest copy (host entry point)
   HostIo* io_ = nullptr;
+  const UnionIn* uni_ = nullptr;  // the input is a union read in place
 
  private:
   // ---- memory
@@ -670,7 +671,8 @@ kamsta_status Solve::pass(int phase, const SegList* src, const uint32_t* map, ui
                           bool validate, bool fetch) {
   const bool dir = src == nullptr;
   const uint64_t total = dir ? md_ : src->total;
-  const int items = (map != nullptr && dir_items_ == 8) ? kMappedDirItems : dir_items_;
+  const int items = uni_ ? kItemsDir
+                    : (map != nullptr && dir_items_ == 8) ? kMappedDirItems : dir_items_;
   int sitems = seg_items_;
   uint32_t smin_n = 0;
   if (!dir && phase == KAMSTA_PHASE_ROUND_EDGES && round_nr_ > 0) {
@@ -686,8 +688,12 @@ kamsta_status Solve::pass(int phase, const SegList* src, const uint32_t* map, ui
                          : rec_dyn_smem(sitems) + round_up(size_t(smin_n) * 8, 16);
   const bool mapped = map != nullptr;
   const bool hub = dir && !mapped && items == 6 && long_rows_ && direct_emit_;
+  const bool uni = dir && uni_ != nullptr;
+  static_assert(kUnionMinGraph > dir_tile(kItemsDir) + 4, "a tile lies in two graphs at most");
   const int per_sm =
-      !dir ? (sitems == 2 ? blocks_per_sm(k_pass_seg<NOUT, 2>, dyn)
+      uni ? (mapped ? blocks_per_sm(k_pass_dir<NOUT, kItemsDir, true, false, true>, dyn)
+                    : blocks_per_sm(k_pass_dir<NOUT, kItemsDir, false, false, true>, dyn))
+      : !dir ? (sitems == 2 ? blocks_per_sm(k_pass_seg<NOUT, 2>, dyn)
               : sitems == 4 ? blocks_per_sm(k_pass_seg<NOUT, 4>, dyn)
                           : blocks_per_sm(k_pass_seg<NOUT, 8>, dyn))
       : mapped ? (items == 8    ? blocks_per_sm(k_pass_dir<NOUT, 8, true>, dyn)
@@ -737,6 +743,11 @@ kamsta_status Solve::pass(int phase, const SegList* src, const uint32_t* map, ui
     a.validate = validate ? 1 : 0;
     a.aligned16 = aligned16_ ? 1 : 0;
     a.smin_n = smin_n;
+    if (uni) {
+      a.ug = uni_->graphs;
+      a.ng = uni_->count;
+      a.gerr = uni_->err;
+    }
     const int t0 = tick();
     bool launched = false;
     if (dir && !mapped && !input_complete_ && attempt == 0) {
@@ -766,7 +777,11 @@ kamsta_status Solve::pass(int phase, const SegList* src, const uint32_t* map, ui
     }
     if (launched) {
       // the first pass ran in groups above
-    } else if (dir && mapped && items == 8)
+    } else if (uni && mapped)
+      k_pass_dir<NOUT, kItemsDir, true, false, true><<<G, kBlock, dyn, st_>>>(nullptr, a);
+    else if (uni)
+      k_pass_dir<NOUT, kItemsDir, false, false, true><<<G, kBlock, dyn, st_>>>(nullptr, a);
+    else if (dir && mapped && items == 8)
       k_pass_dir<NOUT, 8, true><<<G, kBlock, dyn, st_>>>(in_, a);
     else if (dir && mapped && items == 6)
       k_pass_dir<NOUT, 6, true><<<G, kBlock, dyn, st_>>>(in_, a);
@@ -1108,6 +1123,9 @@ kamsta_status Solve::sample_weights(const SegList* L, std::vector<uint32_t>* out
   const int tp = tick();
   if (L) {
     k_sample_weights_seg<<<1, kSampleBlock, 0, st_>>>(L->in(), m, cfg_.seed, samples_);
+  } else if (uni_) {
+    k_sample_weights_union<<<1, kSampleBlock, 0, st_>>>(uni_->graphs, uni_->count, m, cfg_.seed,
+                                                        samples_);
   } else {
     k_sample_weights<<<1, kSampleBlock, 0, st_>>>(in_, m, n_, cfg_.seed, samples_);
   }
@@ -1316,7 +1334,7 @@ kamsta_status Solve::contract(const SegList* L, uint32_t wmin, uint32_t wmax, do
     }
   }
   KS_TRY(pick_big(&big_label_, &use_big_));
-  if (!L && use_big_) {  // heaviest class of the directed input: row scans
+  if (!L && use_big_ && !uni_) {  // heaviest class of the directed input: row scans
     SegList* E = new_list();
     bool done = false;
     KS_TRY(contract_rows(wmin, wmax, E, &done));
@@ -1382,7 +1400,7 @@ bool Solve::coop_options() const {
 }
 
 bool Solve::coop_fits() const {
-  return coop_options() && md_ <= kCoopMaxMd && bounds_.size() + 1 <= coop::kMaxLaunch;
+  return coop_options() && !uni_ && md_ <= kCoopMaxMd && bounds_.size() + 1 <= coop::kMaxLaunch;
 }
 
 // One CTA per SM; little work takes fewer, so that its barriers are short.
@@ -1917,6 +1935,12 @@ kamsta_status Solve::run(Algo algo, kamsta_wedge* d_out, SolveOut* out) {
     KAMSTA_DIR_ATTR(1, 6, false, d6);
     KAMSTA_DIR_ATTR(2, 6, false, d6);
     KAMSTA_DIR_ATTR(3, 6, false, d6);
+    CU_TRY(cudaFuncSetAttribute(k_pass_dir<1, kItemsDir, false, false, true>, attr, d6));
+    CU_TRY(cudaFuncSetAttribute(k_pass_dir<2, kItemsDir, false, false, true>, attr, d6));
+    CU_TRY(cudaFuncSetAttribute(k_pass_dir<3, kItemsDir, false, false, true>, attr, d6));
+    CU_TRY(cudaFuncSetAttribute(k_pass_dir<1, kItemsDir, true, false, true>, attr, d6));
+    CU_TRY(cudaFuncSetAttribute(k_pass_dir<2, kItemsDir, true, false, true>, attr, d6));
+    CU_TRY(cudaFuncSetAttribute(k_pass_dir<3, kItemsDir, true, false, true>, attr, d6));
     CU_TRY(cudaFuncSetAttribute(k_pass_dir<1, 6, false, true>, attr, d6));
     CU_TRY(cudaFuncSetAttribute(k_pass_dir<2, 6, false, true>, attr, d6));
     CU_TRY(cudaFuncSetAttribute(k_pass_dir<3, 6, false, true>, attr, d6));
@@ -2030,7 +2054,8 @@ kamsta_status Solve::run(Algo algo, kamsta_wedge* d_out, SolveOut* out) {
 kamsta_status solve_device(kamsta_ctx* ctx, Algo algo, const kamsta_wedge* d_in,
                            uint64_t m_directed, uint32_t n, const kamsta_cfg& cfg,
                            kamsta_wedge* d_out, SolveOut* out, kamsta_stats* st,
-                           cudaStream_t stream, uint32_t* d_forest_bits, HostIo* io) {
+                           cudaStream_t stream, uint32_t* d_forest_bits, HostIo* io,
+                           const UnionIn* uni) {
   if (st) std::memset(st, 0, sizeof(*st));
   const cudaStream_t str = stream ? stream : ctx->stream;
   auto once = [&]() -> kamsta_status {
@@ -2038,6 +2063,7 @@ kamsta_status solve_device(kamsta_ctx* ctx, Algo algo, const kamsta_wedge* d_in,
     Solve s(ctx, str, d_in, m_directed, n, cfg, st);
     s.forest_bits_ = d_forest_bits;
     s.io_ = io;
+    s.uni_ = uni;
     const kamsta_status r = s.run(algo, d_out, out);
     // a solve that ran to its end has waited for its last kernel
     if (r == KAMSTA_OK) scope.finished();

@@ -145,8 +145,23 @@ struct HostIo {
   uint64_t early = 0;  // out
 };
 
+// A union of graphs read in place instead of from one array: device table in
+// entry order and, per graph, whether an id was out of range (set by the
+// solve).  m_directed counts the unused entries between graphs too.  Forest
+// bitmap only; host-driven rounds only.
+struct UnionIn {
+  const UnionGraph* graphs = nullptr;
+  uint32_t count = 0;
+  uint32_t* err = nullptr;
+};
+// The smallest union read in place.  The cooperative rounds end here: they
+// read an array, and win more than the copy costs (0.14 ms at 2^25 entries).
+// Above, the copy only costs.
+constexpr uint64_t kUnionMinMd = 1ull << 25;
+
 // Solves one graph whose directed, (src,dst)-sorted input lies in device
-// memory.  Writes the forest to d_out (device, capacity >= n-1), or, when
+// memory (or, with `uni`, in the graphs of a union; d_in is null then).
+// Writes the forest to d_out (device, capacity >= n-1), or, when
 // d_forest_bits is given (zeroed, one bit per input entry), sets the bit of
 // the src<dst input copy of every forest edge instead (out->weight is then
 // 0: the caller reads the marked entries).
@@ -154,7 +169,7 @@ kamsta_status solve_device(kamsta_ctx* ctx, Algo algo, const kamsta_wedge* d_in,
                            uint64_t m_directed, uint32_t n, const kamsta_cfg& cfg,
                            kamsta_wedge* d_out, SolveOut* out, kamsta_stats* st,
                            cudaStream_t stream, uint32_t* d_forest_bits = nullptr,
-                           HostIo* io = nullptr);
+                           HostIo* io = nullptr, const UnionIn* uni = nullptr);
 
 void set_error(const std::string& msg);
 kamsta_status cuda_status(cudaError_t e, const char* what);

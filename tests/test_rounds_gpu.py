@@ -339,3 +339,58 @@ def test_row_scans_match_the_streamed_class(kamsta, oracle, rows):
     assert k == kw == len(ref) and np.array_equal(got, want)
     ctx.close()
     assert sw["row_scans"] >= 1
+
+
+@pytest.mark.parametrize("filt,lp", [(False, 1), (False, 0), (True, 0)])
+def test_union_read_in_place_matches_the_copied_union(kamsta, filt, lp):
+    """A batch of 2^25 entries or more whose graphs start on 16-byte
+    boundaries is read in place; one graph off such a boundary makes the same
+    batch a copied union.  Entry counts of every remainder mod 4, graphs of
+    little more than a tile between larger ones, one with an id out of range:
+    the same bytes, counts, weights and status."""
+    import torch
+    ctx = kamsta.Context(0)
+    sizes = [(40001, 1540), (40000, 1536), (50021, 1539)] + \
+            [(33000 + 517 * i, 130001 + 1801 * i) for i in range(88)] + [(32769, 1537)]
+    assert 2 * sum(m for _, m in sizes) > (1 << 25) + 4 * len(sizes)
+    bufs, mds = [], []
+    for i, (n, m) in enumerate(sizes):
+        d = torch.zeros((2 * m + 1, 3), dtype=torch.int32, device="cuda")
+        md = ctx.gen_gnm_dev(n, m, 1000 + i, 254, d.data_ptr())
+        # the last entries are the src > dst copies of edges: the solve reads the others
+        mds.append(max(3072, md - i % 4))
+        bufs.append(d)
+    bufs[20][777, 1] = sizes[20][0]  # an id out of range
+    n = [s[0] for s in sizes]
+    runs = []
+    for shift in (0, 1):
+        src = bufs[45]
+        if shift:
+            src = torch.zeros_like(bufs[45])
+            src[1:] = bufs[45][:-1]
+        outs = [torch.full((x, 3), -1, dtype=torch.int32, device="cuda") for x in n]
+        descs = (kamsta.GraphDesc * len(n))()
+        for i in range(len(n)):
+            b = src if i == 45 else bufs[i]
+            descs[i].edges = b.data_ptr() + (12 * shift if i == 45 else 0)
+            descs[i].m_directed, descs[i].n, descs[i].out = mds[i], n[i], outs[i].data_ptr()
+        st = {}
+        torch.cuda.synchronize()
+        ctx.batch_dev(descs, kamsta.AlgorithmConfig(filter=filt, local_preprocessing=lp),
+                      stats=st)
+        torch.cuda.synchronize()
+        runs.append(([(d.status, d.out_count, d.total_weight) for d in descs], outs, st))
+    (a, ao, sa), (b, bo, sb) = runs
+    assert a == b and sa["entries"] == sb["entries"] == sum(mds)
+    assert a[20][0] != 0 and all(x[0] == 0 for i, x in enumerate(a) if i != 20)
+    for i in range(len(n)):
+        if i != 20:
+            assert torch.equal(ao[i], bo[i]), i
+    # three graphs on their own (whole: a single solve wants both copies of an edge)
+    for i in (0, 45, len(n) - 1):
+        o = torch.zeros((n[i], 3), dtype=torch.int32, device="cuda")
+        s1 = {}
+        k = ctx.boruvka_dev(bufs[i].data_ptr(), 2 * sizes[i][1], n[i], o.data_ptr(),
+                            kamsta.AlgorithmConfig(local_preprocessing=1), stats=s1)
+        assert (k, s1["total_weight"]) == a[i][1:]
+    ctx.close()
