@@ -481,65 +481,6 @@ __device__ void write_phase(Shared& s, const Args& a, uint32_t n, const uint64_t
   }
 }
 
-// Label of every vertex from its tagged root (k_jump_label).
-__device__ void label_phase(const Args& a, uint32_t n, uint32_t* label) {
-  uint32_t* parent = a.parent;
-  const uint32_t stride = gridDim.x * kThreads;
-  auto decode = [](uint32_t t) { return t == kRootTagNone ? kNone : (t & ~kRootTag); };
-  for (uint64_t base = blockIdx.x * kThreads + threadIdx.x; base < n;
-       base += uint64_t(kItems) * stride) {
-    uint32_t x[kItems], p[kItems], lab[kItems];
-    bool run[kItems];
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-      const uint64_t v = base + uint64_t(k) * stride;
-      x[k] = static_cast<uint32_t>(v);
-      p[k] = v < n ? ld_weak_u32(parent + v) : kRootTagNone;
-      run[k] = !(p[k] & kRootTag);
-      lab[k] = run[k] ? kNone : decode(p[k]);
-    }
-    uint32_t steps = 0;
-    for (;;) {
-      bool any = false;
-      uint32_t gp[kItems];
-#pragma unroll
-      for (int k = 0; k < kItems; ++k) gp[k] = run[k] ? ld_weak_u32(parent + p[k]) : 0u;
-#pragma unroll
-      for (int k = 0; k < kItems; ++k) {
-        if (!run[k]) continue;
-        if (gp[k] & kRootTag) {
-          lab[k] = decode(gp[k]);
-          run[k] = false;
-          continue;
-        }
-        st_relaxed(parent + x[k], gp[k]);  // halving
-        x[k] = gp[k];
-        any = true;
-      }
-      if (!any) break;
-#pragma unroll
-      for (int k = 0; k < kItems; ++k) {
-        if (!run[k]) continue;
-        p[k] = ld_weak_u32(parent + x[k]);
-        if (p[k] & kRootTag) {
-          lab[k] = decode(p[k]);
-          run[k] = false;
-        }
-      }
-      ++steps;
-      if ((steps & 1023u) == 0 && (steps > kJumpCap || (ld_relaxed(a.err) & kErrJump))) {
-        atomicOr(a.err, kErrJump);
-        break;
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-      const uint64_t v = base + uint64_t(k) * stride;
-      if (v < n) label[v] = lab[k];
-    }
-  }
-}
-
 // Vertex work of a round over n <= kTinyN vertices, by every CTA in its own
 // shared memory; leaves the label map in s.map.  CTA 0 writes the round's
 // map, the representatives and the forest edges.  Returns the next round's
@@ -720,7 +661,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_rounds(const __grid_constant__ 
       write_phase(s, a, nr, minv, orig_cur, orig_next, min_next, a.n + 64 - ooff, msf_count,
                   direct);
       if (!grid_sync(s, bar, goal, a.err)) return;
-      label_phase(a, nr, R);
+      label_walks<kItems>(nr, gtid, gsz, a.parent, R, a.err);
       const bool to_tiny = n_next <= kTinyN;
       if (to_tiny) {
         for (uint32_t x = tid; x < n_next; x += kThreads) s.min64[x] = kInf64;

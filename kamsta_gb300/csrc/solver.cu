@@ -995,8 +995,12 @@ kamsta_status Solve::rounds(SegList* L, bool own) {
     }
     va.root_tag = tagged ? parent_ : nullptr;
     k_vertex_write<<<gvs, kBlock, 0, st_>>>(va);
-    if (tagged) k_jump_label<<<gv, kBlock, 0, st_>>>(nr, parent_, R, ctx_->d_err);
-    else k_map<<<gv, kBlock, 0, st_>>>(nr, minv, newid_, R);
+    if (tagged) {
+      // (no more CTAs than run at once: a walk waits for none, but skips
+      // ahead only where the walks of other CTAs have begun)
+      const int gj = std::min(gv, blocks_per_sm(k_jump_label, 0) * sms_);
+      k_jump_label<<<gj, kBlock, 0, st_>>>(nr, parent_, R, ctx_->d_err);
+    } else k_map<<<gv, kBlock, 0, st_>>>(nr, minv, newid_, R);
     tock(KAMSTA_PHASE_ROUND_VERTS, tv);
     // relabel + self-loop removal + compaction + next-round minimum
     SegList* nxt = new_list();

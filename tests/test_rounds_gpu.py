@@ -394,3 +394,26 @@ def test_union_read_in_place_matches_the_copied_union(kamsta, filt, lp):
                             kamsta.AlgorithmConfig(local_preprocessing=1), stats=s1)
         assert (k, s1["total_weight"]) == a[i][1:]
     ctx.close()
+
+
+@pytest.mark.parametrize("n,trace", [(4097, False), (300007, False), (300007, True),
+                                     ((1 << 22) + 3, True), ((1 << 24) + 5, False)])
+@pytest.mark.parametrize("falling", [False, True])
+def test_one_hook_chain_through_all_vertices(kamsta, n, trace, falling):
+    """A path whose weights rise or fall along it hooks into one chain: the
+    label walks are taken up in turns, and the forest is the whole path."""
+    import torch
+    i = torch.arange(n - 1, device="cuda", dtype=torch.int32)
+    w = (n - i) if falling else (i + 1)
+    e = torch.empty((2 * (n - 1), 3), dtype=torch.int32, device="cuda")
+    e[0::2] = torch.stack([i, i + 1, w], 1)  # (i, i+1) and (i+1, i), sorted by (src, dst)
+    e[1::2] = torch.stack([i + 1, i, w], 1)
+    o = torch.zeros((n, 3), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ctx, st = kamsta.Context(0), {}
+    k = ctx.boruvka_dev(e.data_ptr(), len(e), n, o.data_ptr(),
+                        kamsta.AlgorithmConfig(trace=trace), stats=st)
+    assert k == n - 1 and st["total_weight"] == int(w.to(torch.int64).sum())
+    got = o[:k][torch.argsort(o[:k, 0])]
+    assert torch.equal(got, e[0::2])
+    ctx.close()
