@@ -131,6 +131,10 @@ HeapScope::HeapScope(kamsta_ctx* ctx, cudaStream_t st) : ctx_(ctx), st_(st) {
   h.st = st;
   h.live = 0;
   // nothing of the heap is in use now; grow by replacing it
+  if (!h.off && h.want > h.cap) {
+    const size_t more = std::max(h.want, h.cap + h.cap / 4);
+    if (!ctx->mem_limit || ctx_device_bytes(ctx) - h.cap + more <= ctx->mem_limit) h.want = more;
+  }
   if (!h.off && h.want > h.cap &&
       (!ctx->mem_limit || ctx_device_bytes(ctx) - h.cap + h.want <= ctx->mem_limit)) {
     heap_release(ctx);

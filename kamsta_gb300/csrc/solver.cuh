@@ -42,7 +42,8 @@ struct Arena {
 // with the heap).
 // A call opens the heap for its stream (HeapScope): blocks taken and given
 // back inside are reused in that stream's order only.  The block grows
-// between calls to what the largest call so far had live at once.
+// between calls to what the largest call so far had live at once, by a
+// quarter at least: its release waits for the whole device.
 struct Heap {
   struct Region {
     size_t off, size;
