@@ -876,6 +876,7 @@ static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_de
 kamsta_status solve_wave(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint32_t G,
                          const kamsta_cfg& cfg, bool host_buffers, cudaStream_t st,
                          BatchWaveStats* ws) {
+  InFlight in_flight(ctx);
   auto once = [&]() -> kamsta_status {
     HeapScope scope(ctx, st);
     const kamsta_status s = solve_wave_once(ctx, algo, g, G, cfg, host_buffers, st, ws);

@@ -17,6 +17,7 @@
 // Edge lists are segmented (see kernels.cuh): every edge pass writes one
 // segment per CTA, so no pass has a cross-CTA scan on its critical path.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -392,6 +393,8 @@ class Solve {
   kamsta_status coop_launch(coop::Args a);
   kamsta_status coop_buffers(uint64_t cap, SegList* reuse);
   bool coop_options() const;  // the solve's options allow cooperative rounds
+  // and few other solves are on the device now (InFlight)
+  bool coop_now() const { return coop_options() && InFlight::few(ctx_->device); }
   // All rounds left of a contraction whose list has become small enough, and
   // (whole contractions over few vertices) the label update; false in *ran
   // when there is no memory for the buffers.
@@ -934,7 +937,7 @@ kamsta_status Solve::rounds(SegList* L, bool own) {
   uint32_t& r = rs.r;
   bool finalized = false;
   while (cur->total > 0) {
-    if (coop_options() && cur->total <= kTailM && nr <= kTailN) {
+    if (coop_now() && cur->total <= kTailM && nr <= kTailN) {
       bool ran = false;
       KS_TRY(coop_tail(cur, cur_owned, false, &rs, &ran, &finalized));
       if (ran) break;
@@ -1323,7 +1326,7 @@ kamsta_status Solve::contract_rows(uint32_t wmin, uint32_t wmax, SegList* E, boo
 kamsta_status Solve::contract(const SegList* L, uint32_t wmin, uint32_t wmax, double frac) {
   if ((L && L->total == 0) || nreps_ <= 1) return KAMSTA_OK;
   fill_inf(minA_, nreps_);
-  if (L && coop_options() && L->total <= kTailM && n_ <= kTailN) {
+  if (L && coop_now() && L->total <= kTailM && n_ <= kTailN) {
     // relabelled, contracted and finished by one cooperative launch; its
     // labels lie in the L2, so no membership bitmap is needed
     Rounds rs;
@@ -1408,7 +1411,7 @@ bool Solve::coop_options() const {
 }
 
 bool Solve::coop_fits() const {
-  return coop_options() && !uni_ && md_ <= kCoopMaxMd && bounds_.size() + 1 <= coop::kMaxLaunch;
+  return coop_now() && !uni_ && md_ <= kCoopMaxMd && bounds_.size() + 1 <= coop::kMaxLaunch;
 }
 
 // One CTA per SM; little work takes fewer, so that its barriers are short.
@@ -2059,12 +2062,33 @@ kamsta_status Solve::run(Algo algo, kamsta_wedge* d_out, SolveOut* out) {
   return KAMSTA_OK;
 }
 
+namespace {
+constexpr int kCountedDevices = 64;
+constexpr int kCoopSolves = 2;
+std::atomic<int> g_in_flight[kCountedDevices];
+}  // namespace
+
+InFlight::InFlight(kamsta_ctx* ctx) : ctx_(ctx) {
+  if (ctx_->solves++ == 0 && ctx_->device >= 0 && ctx_->device < kCountedDevices)
+    g_in_flight[ctx_->device].fetch_add(1);
+}
+
+InFlight::~InFlight() {
+  if (--ctx_->solves == 0 && ctx_->device >= 0 && ctx_->device < kCountedDevices)
+    g_in_flight[ctx_->device].fetch_sub(1);
+}
+
+bool InFlight::few(int device) {
+  return device >= 0 && device < kCountedDevices && g_in_flight[device].load() <= kCoopSolves;
+}
+
 kamsta_status solve_device(kamsta_ctx* ctx, Algo algo, const kamsta_wedge* d_in,
                            uint64_t m_directed, uint32_t n, const kamsta_cfg& cfg,
                            kamsta_wedge* d_out, SolveOut* out, kamsta_stats* st,
                            cudaStream_t stream, uint32_t* d_forest_bits, HostIo* io,
                            const UnionIn* uni) {
   if (st) std::memset(st, 0, sizeof(*st));
+  InFlight in_flight(ctx);
   const cudaStream_t str = stream ? stream : ctx->stream;
   auto once = [&]() -> kamsta_status {
     HeapScope scope(ctx, str);
