@@ -152,12 +152,12 @@ typedef void* kamsta_stream; /* a cudaStream_t; NULL = the context's stream */
 
 kamsta_status kamsta_ctx_create(int device, kamsta_ctx** out);
 kamsta_status kamsta_ctx_destroy(kamsta_ctx* ctx);
-/* Releases cached scratch memory of the context. */
+/* Releases cached scratch memory of the context (arenas, heap and pool). */
 kamsta_status kamsta_ctx_trim(kamsta_ctx* ctx);
-/* Device bytes currently held by the context's scratch pool. */
+/* Device bytes currently held by the context's scratch pool and heap. */
 uint64_t kamsta_ctx_pool_bytes(const kamsta_ctx* ctx);
 /* Caps the device bytes the context may have in use (live allocations of
- * its scratch pool plus its arenas); 0 = no cap (the default).  A call that
+ * its scratch pool plus its arenas and heap); 0 = no cap (the default).  A call that
  * would go over it fails with KAMSTA_E_OOM and leaves the context usable,
  * like a failed device allocation. */
 kamsta_status kamsta_ctx_set_memory_limit(kamsta_ctx* ctx, uint64_t bytes);
@@ -186,8 +186,7 @@ kamsta_status kamsta_mst_boruvka_wedge64(const kamsta_wedge64* edges,
 
 /* ---- single-graph solve, device buffers --------------------------------
  * d_edges / d_out are device pointers; the call is stream-ordered on
- * `stream` and returns after the result count is known (one host read per
- * Boruvka round).  out_count and stats are host pointers.                   */
+ * `stream` and returns after the result count is known.  out_count and stats are host pointers.                   */
 kamsta_status kamsta_mst_boruvka_dev(kamsta_ctx* ctx, const kamsta_wedge* d_edges,
                                      uint64_t m_directed, uint32_t n,
                                      const kamsta_cfg* cfg, kamsta_wedge* d_out,
@@ -265,7 +264,8 @@ kamsta_status kamsta_mst_batch(kamsta_ctx* ctx, kamsta_graph_desc* graphs, uint3
                                kamsta_batch_stats* stats);
 
 /* Batch tuning of a context: the CTA size of the persistent small-graph
- * kernel (256, 512 or 1024 threads) and the largest n it takes (4096 ..
+ * kernel's middle size class (256, 512 or 1024 threads; smaller graphs take
+ * 128, larger ones 1024) and the largest n it takes (4096 ..
  * 32768; larger graphs go to the union solve).  kamsta_batch_autotune times
  * every candidate on the given sample of graphs (device buffers; their
  * outputs are written as by kamsta_mst_batch_dev), keeps the fastest in the
