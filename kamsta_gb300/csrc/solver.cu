@@ -103,7 +103,10 @@ bool Heap::give(void* p) {
 
 void heap_release(kamsta_ctx* ctx) {
   Heap& h = ctx->heap;
-  if (h.base) cudaFree(h.base);
+  if (h.base) {
+    cudaFreeAsync(h.base, ctx->stream);
+    cudaStreamSynchronize(ctx->stream);
+  }
   h.base = nullptr;
   h.cap = 0;
   h.free_list.clear();
@@ -133,15 +136,20 @@ HeapScope::HeapScope(kamsta_ctx* ctx, cudaStream_t st) : ctx_(ctx), st_(st) {
   h.live = 0;
   // nothing of the heap is in use now; grow by replacing it
   if (!h.off && h.want > h.cap) {
-    const size_t more = std::max(h.want, h.cap + h.cap / 4);
+    const size_t more = std::max(h.want + h.want / 8, h.cap + h.cap / 4);
     if (!ctx->mem_limit || ctx_device_bytes(ctx) - h.cap + more <= ctx->mem_limit) h.want = more;
   }
   if (!h.off && h.want > h.cap &&
       (!ctx->mem_limit || ctx_device_bytes(ctx) - h.cap + h.want <= ctx->mem_limit)) {
     heap_release(ctx);
-    if (ctx->pool) cudaMemPoolTrimTo(ctx->pool, 0);
     void* p = nullptr;
-    if (cudaMalloc(&p, h.want) == cudaSuccess) {
+    cudaError_t e = cudaMallocFromPoolAsync(&p, h.want, ctx->pool, st);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      cudaMemPoolTrimTo(ctx->pool, 0);
+      e = cudaMallocFromPoolAsync(&p, h.want, ctx->pool, st);
+    }
+    if (e == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess) {
       h.base = static_cast<char*>(p);
       h.cap = h.want;
     } else {
@@ -167,7 +175,7 @@ HeapScope::~HeapScope() {
 uint64_t ctx_device_bytes(const kamsta_ctx* ctx) {
   uint64_t used = 0;
   if (ctx->pool) cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used);
-  return used + ctx->fixed.cap + ctx->io.cap + ctx->heap.cap;
+  return used + ctx->fixed.cap + ctx->io.cap;  // the heap is from the pool
 }
 
 cudaError_t ctx_alloc(kamsta_ctx* ctx, void** p, size_t bytes, cudaStream_t st) {
