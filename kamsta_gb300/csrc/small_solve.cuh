@@ -374,7 +374,8 @@ __device__ bool solve_keys(const uint32_t* __restrict__ in, uint32_t md, uint32_
         *(heavy[j] ? H - 1 - slot[j] : L[0] + slot[j]) = e[j];
     }
   }
-  if (check_ids && id_max >= n) flag_err(kErrRange);
+  // (without entries id_max is no id: an empty graph of no vertices is valid)
+  if (check_ids && md != 0 && id_max >= n) flag_err(kErrRange);
   if (check_order)
     for (uint32_t i = tid + 1; i < md; i += THREADS) {
       const uint32_t* p = in + 3ull * (i - 1);

@@ -167,3 +167,30 @@ def test_autotune_keeps_results(kamsta):
     torch.cuda.synchronize()
     assert all(np.array_equal(ref[i], outs[i][:descs[i].out_count].cpu().numpy())
                for i in range(len(specs)))
+
+
+def test_batch_dev_takes_graphs_without_edges(kamsta, oracle):
+    """Graphs of 0, 1 and 7 vertices and no entry are valid and have an empty
+    forest, alone and beside others; entries of a graph of no vertices are
+    out of range."""
+    import torch
+    ctx = kamsta.Context(0)
+    e = oracle.gen_gnm(300, 2000, 5)
+    d = torch.from_numpy(e.view(np.uint32).reshape(-1, 3).view(np.int32)).cuda()
+    o = torch.zeros((300, 3), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    for sizes in [(0,), (1,), (7,), (0, 1, 7, 300, 0)]:
+        descs = (kamsta.GraphDesc * len(sizes))()
+        for k, n in enumerate(sizes):
+            descs[k].n, descs[k].out = n, o.data_ptr()
+            if n == 300:
+                descs[k].edges, descs[k].m_directed = d.data_ptr(), len(e)
+        ctx.batch_dev(descs)
+        for k, n in enumerate(sizes):
+            assert descs[k].status == 0
+            assert descs[k].out_count == (len(_sorted_ref(oracle, e, n)[0]) if n == 300 else 0)
+    bad = (kamsta.GraphDesc * 1)()
+    bad[0].n, bad[0].edges, bad[0].m_directed = 0, d.data_ptr(), len(e)
+    ctx.batch_dev(bad)
+    assert bad[0].status == kamsta._native.E_INPUT and bad[0].out_count == 0
+    ctx.close()

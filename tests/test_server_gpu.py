@@ -218,3 +218,16 @@ def test_worker_share_is_the_job_limit(kamsta):
         srv.submit(d.data_ptr(), md, n, out.data_ptr())
     assert ei.value.status == kamsta._native.E_BUDGET
     srv.close()
+
+
+def test_jobs_without_edges(kamsta):
+    import torch
+    out = torch.zeros((8, 3), dtype=torch.int32, device="cuda")
+    srv = kamsta.Server(0, budget_bytes=1 << 30, workers=1)
+    for n in (0, 1, 7):
+        srv.submit(0, 0, n, out.data_ptr(), tag=n)
+    got = _drain(srv, 3)
+    srv.close()
+    for n in (0, 1, 7):
+        assert got[n]["status"] == 0
+        assert got[n]["out_count"] == 0 and got[n]["total_weight"] == 0
