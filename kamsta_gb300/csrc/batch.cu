@@ -500,10 +500,11 @@ cudaError_t launch_small_kernel(int c, int threads, const SmallTable& t, unsigne
 
 // Launches the small graphs, each size class on a stream of its own between
 // `st` and `st`, and returns; `res` (host) is valid after st synchronises.
-// Device buffers stay alive in tab and scr.
+// Device buffers stay alive in tab and scr.  all_full: every graph in the
+// largest class.
 kamsta_status launch_small(kamsta_ctx* ctx, kamsta_graph_desc* g, const std::vector<uint32_t>& idx,
-                           const kamsta_cfg& cfg, cudaStream_t st, PoolBuf* tab, PoolBuf* scr,
-                           small::Result** d_res, uint32_t* launches) {
+                           const kamsta_cfg& cfg, bool all_full, cudaStream_t st, PoolBuf* tab,
+                           PoolBuf* scr, small::Result** d_res, uint32_t* launches) {
   const uint32_t S = static_cast<uint32_t>(idx.size());
   // by class, each by descending work to an eighth of its power of two (the
   // queue only wants the long ones first): one counting sort
@@ -513,7 +514,7 @@ kamsta_status launch_small(kamsta_ctx* ctx, kamsta_graph_desc* g, const std::vec
   uint32_t count[kClasses] = {0, 0, 0};
   for (uint32_t i = 0; i < S; ++i) {
     const kamsta_graph_desc& d = g[idx[i]];
-    const int c = size_class(d);
+    const int c = all_full ? kClasses - 1 : size_class(d);
     ++count[c];
     const uint32_t work = static_cast<uint32_t>(d.m_directed) + d.n + 8;
     const uint32_t lg = 31u - static_cast<uint32_t>(__builtin_clz(work));
@@ -831,7 +832,7 @@ static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_de
   PoolBuf tab, scr;
   small::Result* d_res = nullptr;
   uint32_t launches = 0;
-  B_KTRY(launch_small(ctx, g, sm, cfg, ctx->aux, &tab, &scr, &d_res, &launches));
+  B_KTRY(launch_small(ctx, g, sm, cfg, false, ctx->aux, &tab, &scr, &d_res, &launches));
   BatchWaveStats us;
   kamsta_status s = KAMSTA_OK;
   if (!lg.empty()) {
@@ -851,11 +852,7 @@ static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_de
   B_TRY(cudaStreamSynchronize(ctx->aux));
   if (s != KAMSTA_OK) return s;
   uint64_t entries = 0, verts = 0;
-  for (size_t k = 0; k < sm.size(); ++k) {
-    kamsta_graph_desc& d = g[sm[k]];
-    const small::Result& r = h_res[k];
-    entries += d.m_directed;
-    verts += d.n;
+  auto report = [](kamsta_graph_desc& d, const small::Result& r) {
     if (r.err) {
       d.status = (r.err & ~(kErrRange | kErrOrder)) ? KAMSTA_E_NOCONVERGE : KAMSTA_E_INPUT;
       d.out_count = 0;
@@ -865,6 +862,24 @@ static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_de
       d.out_count = r.count;
       d.total_weight = r.weight;
     }
+  };
+  std::vector<uint32_t> again;
+  for (size_t k = 0; k < sm.size(); ++k) {
+    kamsta_graph_desc& d = g[sm[k]];
+    entries += d.m_directed;
+    verts += d.n;
+    report(d, h_res[k]);
+    if ((h_res[k].err & kErrOverflow) && size_class(d) < kClasses - 1) again.push_back(sm[k]);
+  }
+  if (!again.empty()) {
+    // edges listed in one direction only can be more than a class's lists
+    // hold: those graphs once more in the largest class
+    B_KTRY(launch_small(ctx, g, again, cfg, true, ctx->aux, &tab, &scr, &d_res, &launches));
+    h_res.resize(again.size());
+    B_TRY(cudaMemcpyAsync(h_res.data(), d_res, sizeof(small::Result) * again.size(),
+                          cudaMemcpyDeviceToHost, ctx->aux));
+    B_TRY(cudaStreamSynchronize(ctx->aux));
+    for (size_t k = 0; k < again.size(); ++k) report(g[again[k]], h_res[k]);
   }
   ws->entries = us.entries + entries;
   ws->vertices = us.vertices + verts;

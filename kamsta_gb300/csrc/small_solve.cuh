@@ -38,7 +38,6 @@ namespace small {
 
 constexpr uint32_t kMaxN = 1u << 15;
 constexpr uint64_t kMaxMd = 1ull << 18;
-constexpr uint32_t kMaxMu = static_cast<uint32_t>(kMaxMd / 2);  // src<dst copies
 constexpr uint32_t kMaxRounds = 40;
 // Size classes of the batch: a graph that needs little shared memory and has
 // little work goes to a small CTA, several of which share an SM.
@@ -72,7 +71,8 @@ struct Slot {
 };
 constexpr Slot slot_layout(uint64_t md, uint32_t n) {
   Slot s{};
-  const size_t mu = md / 2 < 256 ? 256 : md / 2;  // (non-symmetric input may overflow it)
+  // (an input that lists edges in one direction only may overflow it: kErrOverflow)
+  const size_t mu = md / 2 < 256 ? 256 : md / 2;
   s.l0 = 256;                                     // Result
   s.l1 = s.l0 + mu * 16;
   s.gmin = s.l1 + mu * 16;

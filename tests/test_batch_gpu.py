@@ -194,3 +194,26 @@ def test_batch_dev_takes_graphs_without_edges(kamsta, oracle):
     ctx.batch_dev(bad)
     assert bad[0].status == kamsta._native.E_INPUT and bad[0].out_count == 0
     ctx.close()
+
+
+@pytest.mark.parametrize("n,m", [(1000, 8193), (1024, 16384), (4096, 16385), (4000, 32769),
+                                 (4096, 65536), (32768, 65537), (32768, 131072)])
+def test_batch_dev_small_graph_listed_in_one_direction(kamsta, oracle, n, m):
+    """Only the src < dst copies: up to 131072 of them are solved, in whichever
+    size class n and the number of entries put the graph."""
+    import torch
+    e = oracle.gen_gnm(n, m, 17)
+    half = e[e["src"] < e["dst"]]
+    d = torch.from_numpy(half.view(np.uint32).reshape(-1, 3).view(np.int32)).cuda()
+    o = torch.zeros((n, 3), dtype=torch.int32, device="cuda")
+    ctx, descs = kamsta.Context(0), (kamsta.GraphDesc * 1)()
+    descs[0].edges, descs[0].m_directed, descs[0].n = d.data_ptr(), len(half), n
+    descs[0].out = o.data_ptr()
+    torch.cuda.synchronize()
+    ctx.batch_dev(descs)
+    ref, w = _sorted_ref(oracle, e, n)
+    assert descs[0].status == 0 and descs[0].out_count == len(ref)
+    assert descs[0].total_weight == w
+    got = o[:len(ref)].cpu().numpy().view(np.uint32).reshape(-1).view(kamsta.WEDGE)
+    assert np.array_equal(got, ref)
+    ctx.close()
