@@ -162,6 +162,14 @@ uint64_t kamsta_ctx_pool_bytes(const kamsta_ctx* ctx);
  * like a failed device allocation. */
 kamsta_status kamsta_ctx_set_memory_limit(kamsta_ctx* ctx, uint64_t bytes);
 
+/* Failure injection for tests of the error paths, on the host alone: the
+ * nth operation of the kind `what` from now fails once without having run
+ * (0 = none).  *pending (may be NULL) receives what was left of the count
+ * set before: 0 when that failure has happened. */
+#define KAMSTA_FAIL_SMALL_LAUNCH 0u /* a launch of the batch's small-graph kernels */
+kamsta_status kamsta_ctx_fail_nth(kamsta_ctx* ctx, uint32_t what, uint32_t nth,
+                                  uint32_t* pending);
+
 /* ---- single-graph solve, host buffers ----------------------------------
  * edges: m_directed entries (host memory); out: capacity >= n-1 entries
  * (host memory).  Uses a per-thread default context on the current device.

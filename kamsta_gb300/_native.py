@@ -144,6 +144,7 @@ SIGNATURES = {
     "kamsta_ctx_trim": (I32, [P]),
     "kamsta_ctx_pool_bytes": (U64, [P]),
     "kamsta_ctx_set_memory_limit": (I32, [P, U64]),
+    "kamsta_ctx_fail_nth": (I32, [P, U32, U32, C.POINTER(U32)]),
     "kamsta_mst_boruvka": (I32, [P, U64, U32, C.POINTER(Cfg), P, C.POINTER(U64), C.POINTER(Stats)]),
     "kamsta_mst_filter_boruvka": (I32, [P, U64, U32, C.POINTER(Cfg), P, C.POINTER(U64),
                                         C.POINTER(Stats)]),

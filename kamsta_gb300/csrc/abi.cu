@@ -578,6 +578,18 @@ kamsta_status kamsta_ctx_set_memory_limit(kamsta_ctx* ctx, uint64_t bytes) {
   return KAMSTA_OK;
 }
 
+kamsta_status kamsta_ctx_fail_nth(kamsta_ctx* ctx, uint32_t what, uint32_t nth,
+                                  uint32_t* pending) {
+  if (!ctx || what >= kFailKinds) {
+    set_error("kamsta_ctx_fail_nth: null context or unknown kind");
+    return KAMSTA_E_INPUT;
+  }
+  std::lock_guard<std::mutex> lock(ctx->mu);
+  if (pending) *pending = ctx->fail_in[what];
+  ctx->fail_in[what] = nth;
+  return KAMSTA_OK;
+}
+
 uint64_t kamsta_ctx_pool_bytes(const kamsta_ctx* ctx) {
   if (!ctx) return 0;
   uint64_t pool = 0;

@@ -595,6 +595,8 @@ kamsta_status launch_small(kamsta_ctx* ctx, kamsta_graph_desc* g, const std::vec
     if (on[c] != st) B_TRY(cudaStreamWaitEvent(on[c], ctx->ev_small[0], 0));
     t.order = reinterpret_cast<const uint32_t*>(d + o_order) + first;
     t.G = count[c];
+    if (fail_now(ctx, KAMSTA_FAIL_SMALL_LAUNCH))
+      return cuda_status(cudaErrorLaunchOutOfResources, "launch of the small-graph kernels");
     B_TRY(launch_small_kernel(c, threads, t, scratch, queue + c, grid[c], nullptr, on[c]));
     scratch += grid[c] * slot[c];
     ++*launches;
@@ -818,6 +820,19 @@ kamsta_status solve_union(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint
 
 bool is_small_graph(const kamsta_ctx* ctx, const kamsta_graph_desc& g) { return is_small(ctx, g); }
 
+// Small graphs under way on the context's side streams.  A call that fails
+// midway waits for them: they use scratch that is freed in aux's order, which
+// the size classes' streams may not have joined yet, and the caller's buffers.
+struct SmallInFlight {
+  kamsta_ctx* ctx;
+  bool done = false;
+  ~SmallInFlight() {
+    if (done) return;
+    for (cudaStream_t s : ctx->small_st) cudaStreamSynchronize(s);
+    cudaStreamSynchronize(ctx->aux);
+  }
+};
+
 static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint32_t G,
                                      const kamsta_cfg& cfg, bool host_buffers, cudaStream_t st,
                                      BatchWaveStats* ws) {
@@ -830,6 +845,7 @@ static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_de
   B_TRY(cudaEventRecord(ctx->ev_fork, st));
   B_TRY(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
   PoolBuf tab, scr;
+  SmallInFlight under_way{ctx};
   small::Result* d_res = nullptr;
   uint32_t launches = 0;
   B_KTRY(launch_small(ctx, g, sm, cfg, false, ctx->aux, &tab, &scr, &d_res, &launches));
@@ -881,6 +897,7 @@ static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_de
     B_TRY(cudaStreamSynchronize(ctx->aux));
     for (size_t k = 0; k < again.size(); ++k) report(g[again[k]], h_res[k]);
   }
+  under_way.done = true;
   ws->entries = us.entries + entries;
   ws->vertices = us.vertices + verts;
   ws->launches = us.launches + launches;

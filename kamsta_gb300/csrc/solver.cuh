@@ -82,6 +82,7 @@ constexpr int kTimerEvents = 64;
 constexpr uint32_t kCountWords = 3 * 1024;  // segment counts of a pass's outputs
 constexpr size_t kHostState = 1024;  // bytes of kamsta_ctx::h_state
 constexpr int kInputPieces = 16;  // host input copied in this many pieces
+constexpr uint32_t kFailKinds = 1;  // KAMSTA_FAIL_*
 
 }  // namespace kamsta
 
@@ -119,6 +120,7 @@ struct kamsta_ctx {
   cudaEvent_t ev_early = nullptr;  // the first round's forest edges are written
   uint64_t mem_limit = 0;          // kamsta_ctx_set_memory_limit; 0 = none
   int solves = 0;        // nested InFlight scopes (under mu)
+  uint32_t fail_in[kamsta::kFailKinds] = {};  // kamsta_ctx_fail_nth; 0 = off
   std::mutex mu;
 };
 
@@ -195,6 +197,12 @@ kamsta_status solve_device(kamsta_ctx* ctx, Algo algo, const kamsta_wedge* d_in,
                            kamsta_wedge* d_out, SolveOut* out, kamsta_stats* st,
                            cudaStream_t stream, uint32_t* d_forest_bits = nullptr,
                            HostIo* io = nullptr, const UnionIn* uni = nullptr);
+
+// Whether the operation of this kind that is about to run is the one to fail.
+inline bool fail_now(kamsta_ctx* ctx, uint32_t what) {
+  uint32_t& in = ctx->fail_in[what];
+  return in != 0 && --in == 0;
+}
 
 void set_error(const std::string& msg);
 kamsta_status cuda_status(cudaError_t e, const char* what);
