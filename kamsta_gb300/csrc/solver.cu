@@ -178,6 +178,20 @@ uint64_t ctx_device_bytes(const kamsta_ctx* ctx) {
   return used + ctx->fixed.cap + ctx->io.cap;  // the heap is from the pool
 }
 
+// A request to the pool.  A failed one leaves no error behind in the runtime:
+// callers that can do without the memory go on, and what they launch next asks
+// for the last error.
+static cudaError_t pool_alloc(kamsta_ctx* ctx, void** p, size_t bytes, cudaStream_t st) {
+  const cudaError_t e = fail_now(ctx, KAMSTA_FAIL_POOL_ALLOC)
+                            ? cudaMalloc(p, size_t(1) << 60)  // as when the device is full
+                            : cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+  }
+  return e;
+}
+
 cudaError_t ctx_alloc(kamsta_ctx* ctx, void** p, size_t bytes, cudaStream_t st) {
   *p = nullptr;
   Heap& h = ctx->heap;
@@ -192,7 +206,7 @@ cudaError_t ctx_alloc(kamsta_ctx* ctx, void** p, size_t bytes, cudaStream_t st) 
   }
   if (ctx->mem_limit && ctx_device_bytes(ctx) + bytes > ctx->mem_limit)
     return cudaErrorMemoryAllocation;
-  const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+  const cudaError_t e = pool_alloc(ctx, p, bytes, st);
   if (open && e == cudaSuccess) h.pooled.push_back({*p, (bytes + 255) & ~static_cast<size_t>(255)});
   return e;
 }
@@ -1612,6 +1626,7 @@ kamsta_status Solve::coop_tail(SegList* L, bool own, bool prologue, Rounds* R, b
     return coop_reset();
   }();
   if (s == KAMSTA_E_OOM) {
+    for (SegList* B : coop_list_) free_list(B);
     coop_off_ = true;
     *finalized = false;
     return KAMSTA_OK;

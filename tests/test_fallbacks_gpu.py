@@ -8,7 +8,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SMALL_LAUNCH = 0
+SMALL_LAUNCH, POOL_ALLOC = 0, 1
 
 
 def _fail(kamsta, ctx, what, nth):
@@ -65,3 +65,50 @@ def _sorted_forest(oracle, edges, n):
     t = f.copy()
     t["src"], t["dst"] = np.minimum(f["src"], f["dst"]), np.maximum(f["src"], f["dst"])
     return t[np.lexsort((t["dst"], t["src"]))]
+
+
+def _solve(kamsta, ctx, d, md, n, fn, cfg):
+    import torch
+    o = torch.zeros((n, 3), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    k = getattr(ctx, fn)(d.data_ptr(), md, n, o.data_ptr(), cfg)
+    return o[:k].cpu().numpy()
+
+
+@pytest.mark.parametrize("n,m,fn,lp,without", [
+    (1000, 4000, "boruvka_dev", 0, 1),       # one CTA: its scratch
+    (20000, 90000, "boruvka_dev", 0, 3),     # cooperative rounds: lists and state
+    (20000, 200000, "boruvka_dev", 1, 3),
+    (20000, 200000, "filter_boruvka_dev", 0, 3),  # each contraction's tail
+    (1 << 20, 17 << 20, "boruvka_dev", 0, 3)])    # the forest first, then its edges
+def test_every_scratch_request_may_fail(kamsta, n, m, fn, lp, without):
+    """The k-th request to the pool fails, for every k of a new context's
+    solve: the call runs out of memory or gives the same forest, and for
+    at least `without` of them, which only serve speed, it gives the forest;
+    the context then solves as before."""
+    import torch
+    gen = kamsta.Context(0)
+    d = torch.empty((2 * m, 3), dtype=torch.int32, device="cuda")
+    md = gen.gen_gnm_dev(n, m, 11, 254, d.data_ptr())
+    cfg = kamsta.AlgorithmConfig(local_preprocessing=lp)
+    want = _solve(kamsta, gen, d, md, n, fn, cfg)
+    done_without = 0
+    for k in range(1, 200):
+        ctx = kamsta.Context(0)
+        _fail(kamsta, ctx, POOL_ALLOC, k)
+        got = None
+        try:
+            got = _solve(kamsta, ctx, d, md, n, fn, cfg)
+        except kamsta.KamstaError as e:
+            assert e.status == kamsta._native.E_OOM
+        unused = _fail(kamsta, ctx, POOL_ALLOC, 0)
+        assert got is not None or unused == 0
+        if got is not None:
+            assert np.array_equal(got, want)
+            done_without += unused == 0
+        assert np.array_equal(_solve(kamsta, ctx, d, md, n, fn, cfg), want)
+        ctx.close()
+        if unused:
+            break
+    assert unused and done_without >= without
+    gen.close()
