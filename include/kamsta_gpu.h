@@ -168,6 +168,7 @@ kamsta_status kamsta_ctx_set_memory_limit(kamsta_ctx* ctx, uint64_t bytes);
  * set before: 0 when that failure has happened. */
 #define KAMSTA_FAIL_SMALL_LAUNCH 0u /* a launch of the batch's small-graph kernels */
 #define KAMSTA_FAIL_POOL_ALLOC 1u   /* a request to the pool: device out of memory */
+#define KAMSTA_FAIL_COOP_LAUNCH 2u  /* a cooperative launch: refused */
 kamsta_status kamsta_ctx_fail_nth(kamsta_ctx* ctx, uint32_t what, uint32_t nth,
                                   uint32_t* pending);
 

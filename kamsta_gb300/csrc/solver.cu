@@ -1410,7 +1410,15 @@ cudaError_t launch_in_order(int dev, const void* f, uint32_t grid, uint32_t bloc
   if (!o.ev) e = cudaEventCreateWithFlags(&o.ev, cudaEventDisableTiming);
   else e = cudaStreamWaitEvent(st, o.ev, 0);
   if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(f, dim3(grid), dim3(block), args, smem, st);
-  if (e == cudaSuccess) e = cudaEventRecord(o.ev, st);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return e;  // nothing has run
+  }
+  // (without the event the next launch has nothing to wait for)
+  if (cudaEventRecord(o.ev, st) != cudaSuccess) {
+    cudaGetLastError();
+    e = cudaStreamSynchronize(st);
+  }
   return e;
 }
 }  // namespace
@@ -1524,6 +1532,8 @@ coop::Args Solve::coop_args(const SegList* L) const {
 
 kamsta_status Solve::coop_launch(coop::Args a) {
   void* args[] = {&a};
+  if (fail_now(ctx_, KAMSTA_FAIL_COOP_LAUNCH))
+    return cuda_status(cudaErrorCooperativeLaunchTooLarge, "cooperative launch");
   const int t0 = tick();
   CU_TRY(launch_in_order(ctx_->device, reinterpret_cast<const void*>(&coop::k_rounds), coop_grid_,
                          coop::kThreads, sizeof(coop::Shared), args, st_));
@@ -1625,14 +1635,15 @@ kamsta_status Solve::coop_tail(SegList* L, bool own, bool prologue, Rounds* R, b
     KS_TRY(coop_buffers((L->total + nq - 1) / nq, own ? L : nullptr));
     return coop_reset();
   }();
-  if (s == KAMSTA_E_OOM) {
+  // not run, and nothing of the contraction has changed
+  auto give_up = [&]() -> kamsta_status {
     for (SegList* B : coop_list_) free_list(B);
     coop_off_ = true;
     *finalized = false;
     return KAMSTA_OK;
-  }
+  };
+  if (s == KAMSTA_E_OOM) return give_up();
   KS_TRY(s);
-  *ran = true;
   coop::Args a = coop_args(L);
   a.first = 1;
   a.nr0 = R->nr;
@@ -1646,7 +1657,9 @@ kamsta_status Solve::coop_tail(SegList* L, bool own, bool prologue, Rounds* R, b
   a.weight = dweight_;
   a.prologue = prologue ? 1u : 0u;
   a.finalize = *finalized ? 1u : 0u;
-  KS_TRY(coop_launch(a));
+  // (a grid of all SMs cannot be resident where the process has only a part)
+  if (coop_launch(a) != KAMSTA_OK) return give_up();
+  *ran = true;
   const kamsta_status fs = coop_fetch();
   for (SegList* B : coop_list_) free_list(B);
   KS_TRY(fs);

@@ -82,7 +82,7 @@ constexpr int kTimerEvents = 64;
 constexpr uint32_t kCountWords = 3 * 1024;  // segment counts of a pass's outputs
 constexpr size_t kHostState = 1024;  // bytes of kamsta_ctx::h_state
 constexpr int kInputPieces = 16;  // host input copied in this many pieces
-constexpr uint32_t kFailKinds = 2;  // KAMSTA_FAIL_*
+constexpr uint32_t kFailKinds = 3;  // KAMSTA_FAIL_*
 
 }  // namespace kamsta
 

@@ -8,7 +8,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SMALL_LAUNCH, POOL_ALLOC = 0, 1
+SMALL_LAUNCH, POOL_ALLOC, COOP_LAUNCH = 0, 1, 2
 
 
 def _fail(kamsta, ctx, what, nth):
@@ -112,3 +112,24 @@ def test_every_scratch_request_may_fail(kamsta, n, m, fn, lp, without):
             break
     assert unused and done_without >= without
     gen.close()
+
+
+@pytest.mark.parametrize("n,m,fn,lp", [
+    (20000, 90000, "boruvka_dev", 0), (20000, 200000, "boruvka_dev", 1),
+    (20000, 200000, "filter_boruvka_dev", 0), (1 << 20, 17 << 20, "boruvka_dev", 1)])
+def test_refused_cooperative_launch_is_done_without(kamsta, n, m, fn, lp):
+    """Whichever cooperative launch of a solve is refused, the rounds run
+    host-driven from there (or from the start) and give the same forest."""
+    import torch
+    ctx = kamsta.Context(0)
+    d = torch.empty((2 * m, 3), dtype=torch.int32, device="cuda")
+    md = ctx.gen_gnm_dev(n, m, 12, 254, d.data_ptr())
+    cfg = kamsta.AlgorithmConfig(local_preprocessing=lp)
+    want = _solve(kamsta, ctx, d, md, n, fn, cfg)
+    for k in range(1, 60):
+        _fail(kamsta, ctx, COOP_LAUNCH, k)
+        assert np.array_equal(_solve(kamsta, ctx, d, md, n, fn, cfg), want)
+        if _fail(kamsta, ctx, COOP_LAUNCH, 0):
+            break
+    assert k > 1
+    ctx.close()
