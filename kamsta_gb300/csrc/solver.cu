@@ -113,12 +113,20 @@ void heap_release(kamsta_ctx* ctx) {
   h.used.clear();
 }
 
+// Gives the block back while no call has it open (generators, loaders, the
+// decoder and the io buffers take their memory then).  False when there was
+// nothing to give.
+static bool heap_give_back(kamsta_ctx* ctx) {
+  if (ctx->heap.depth > 0 || ctx->heap.cap == 0) return false;
+  heap_release(ctx);
+  return true;
+}
+
 // After a call that ran out of memory: gives the heap's block back and keeps
 // the context on its pool alone.  True when that can help (nothing of the
 // heap is in use and it held memory).
 bool heap_retry(kamsta_ctx* ctx) {
-  if (ctx->heap.depth > 0 || ctx->heap.cap == 0) return false;
-  heap_release(ctx);
+  if (!heap_give_back(ctx)) return false;
   ctx->heap.off = true;
   ctx->heap.want = 0;
   return true;
@@ -135,26 +143,28 @@ HeapScope::HeapScope(kamsta_ctx* ctx, cudaStream_t st) : ctx_(ctx), st_(st) {
   h.st = st;
   h.live = 0;
   // nothing of the heap is in use now; grow by replacing it
+  auto fits = [&](size_t size) {
+    return !ctx->mem_limit || ctx_device_bytes(ctx) - h.cap + size <= ctx->mem_limit;
+  };
   if (!h.off && h.want > h.cap) {
-    const size_t more = std::max(h.want + h.want / 8, h.cap + h.cap / 4);
-    if (!ctx->mem_limit || ctx_device_bytes(ctx) - h.cap + more <= ctx->mem_limit) h.want = more;
-  }
-  if (!h.off && h.want > h.cap &&
-      (!ctx->mem_limit || ctx_device_bytes(ctx) - h.cap + h.want <= ctx->mem_limit)) {
-    heap_release(ctx);
-    void* p = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(&p, h.want, ctx->pool, st);
-    if (e == cudaErrorMemoryAllocation) {
-      cudaGetLastError();
-      cudaMemPoolTrimTo(ctx->pool, 0);
-      e = cudaMallocFromPoolAsync(&p, h.want, ctx->pool, st);
-    }
-    if (e == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess) {
-      h.base = static_cast<char*>(p);
-      h.cap = h.want;
-    } else {
-      cudaGetLastError();
-      h.want = 0;
+    size_t size = std::max(h.want + h.want / 8, h.cap + h.cap / 4);
+    if (!fits(size)) size = h.want;
+    if (fits(size)) {
+      heap_release(ctx);
+      void* p = nullptr;
+      cudaError_t e = cudaMallocFromPoolAsync(&p, size, ctx->pool, st);
+      if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        cudaMemPoolTrimTo(ctx->pool, 0);
+        e = cudaMallocFromPoolAsync(&p, size, ctx->pool, st);
+      }
+      if (e == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess) {
+        h.base = static_cast<char*>(p);
+        h.cap = size;
+      } else {
+        cudaGetLastError();
+        h.want = 0;
+      }
     }
   }
   h.used.clear();
@@ -204,9 +214,13 @@ cudaError_t ctx_alloc(kamsta_ctx* ctx, void** p, size_t bytes, cudaStream_t st) 
     // enough in all, but in pieces: some room more next time
     if (h.live <= h.cap) h.want = std::max(h.want, h.cap + h.cap / 8 + need / 2);
   }
-  if (ctx->mem_limit && ctx_device_bytes(ctx) + bytes > ctx->mem_limit)
-    return cudaErrorMemoryAllocation;
-  const cudaError_t e = pool_alloc(ctx, p, bytes, st);
+  auto request = [&]() -> cudaError_t {
+    if (ctx->mem_limit && ctx_device_bytes(ctx) + bytes > ctx->mem_limit)
+      return cudaErrorMemoryAllocation;
+    return pool_alloc(ctx, p, bytes, st);
+  };
+  cudaError_t e = request();
+  if (e == cudaErrorMemoryAllocation && heap_give_back(ctx)) e = request();
   if (open && e == cudaSuccess) h.pooled.push_back({*p, (bytes + 255) & ~static_cast<size_t>(255)});
   return e;
 }
@@ -225,13 +239,19 @@ void ctx_free(kamsta_ctx* ctx, void* p, cudaStream_t st) {
 }
 
 cudaError_t ctx_reserve(kamsta_ctx* ctx, Arena& a, size_t bytes) {
-  // growing releases the old buffer first
-  if (bytes > a.cap && ctx->mem_limit &&
-      ctx_device_bytes(ctx) - a.cap + bytes > ctx->mem_limit) {
-    a.reset();
-    return cudaErrorMemoryAllocation;
+  a.reset();
+  auto over = [&] {  // growing releases the old buffer first
+    return bytes > a.cap && ctx->mem_limit &&
+           ctx_device_bytes(ctx) - a.cap + bytes > ctx->mem_limit;
+  };
+  if (over() && !(heap_give_back(ctx) && !over())) return cudaErrorMemoryAllocation;
+  cudaError_t e = a.reserve(bytes);
+  if (e == cudaErrorMemoryAllocation) {  // the pool's cache may hold what is missing
+    heap_give_back(ctx);
+    cudaMemPoolTrimTo(ctx->pool, 0);
+    e = a.reserve(bytes);
   }
-  return a.reserve(bytes);
+  return e;
 }
 
 void Arena::release() {

@@ -53,7 +53,7 @@ struct Heap {
   };
   char* base = nullptr;
   size_t cap = 0;
-  size_t want = 0;                 // size to grow to before the next call
+  size_t want = 0;                 // size the largest call needed
   size_t live = 0;                 // bytes out, here and in the pool, this call
   std::vector<Region> free_list;   // by offset
   std::vector<Region> used;

@@ -133,3 +133,67 @@ def test_refused_cooperative_launch_is_done_without(kamsta, n, m, fn, lp):
             break
     assert k > 1
     ctx.close()
+
+
+def _from_the_heap(kamsta, ctx, solve):
+    """Whether a solve takes nothing from the pool (a request would fail)."""
+    _fail(kamsta, ctx, POOL_ALLOC, 1)
+    try:
+        solve()
+    except kamsta.KamstaError as e:
+        assert e.status == kamsta._native.E_OOM
+    return _fail(kamsta, ctx, POOL_ALLOC, 0) == 1
+
+
+def _least_limit(kamsta, op):
+    """The tightest memory limit, to 2 MB, under which a new context does op."""
+    lo, hi = 1 << 20, 4 << 30
+    while hi - lo > 2 << 20:
+        mid = (lo + hi) // 2
+        c = kamsta.Context(0)
+        c.set_memory_limit(mid)
+        try:
+            op(c)
+            hi = mid
+        except kamsta.KamstaError as e:
+            assert e.status == kamsta._native.E_OOM
+            lo = mid
+        c.close()
+    return hi
+
+
+@pytest.mark.parametrize("what,m_solve", [("7bit", 1450000), ("gnm", 1 << 20),
+                                          ("rgg2d", 1 << 18)])
+def test_idle_scratch_block_gives_way(kamsta, oracle, what, m_solve):
+    """What a new context does under a memory limit it also does after solves
+    that left it a block of scratch: the block is not in use by then."""
+    import torch
+    n, m = 1 << 16, 1 << 20
+    gen = kamsta.Context(0)
+    d = torch.empty((2 * m_solve, 3), dtype=torch.int32, device="cuda")
+    buf = torch.empty((8 * m, 3), dtype=torch.int32, device="cuda")
+    out = torch.empty((n, 3), dtype=torch.int32, device="cuda")
+    md = gen.gen_gnm_dev(n, m_solve, 13, 254, d.data_ptr())
+    small = gen.gen_gnm_dev(n, m, 14, 254, buf.data_ptr())
+    torch.cuda.synchronize()
+    edges = buf[:small].cpu().numpy().view(np.uint32).reshape(-1).view(kamsta.WEDGE)
+    keep, g = gen._cgraph_dev(kamsta.Compressed(edges, n, 4096))
+    op = {"7bit": lambda c: c.boruvka_7bit_dev(g, out.data_ptr()),
+          "gnm": lambda c: c.gen_gnm_dev(n, 2 * m, 14, 254, buf.data_ptr()),
+          "rgg2d": lambda c: c.gen_rgg2d_dev(1 << 20, 0.0012, 15, 254, buf.data_ptr(), 8 * m),
+          }[what]
+    ctx = kamsta.Context(0)
+    solve = lambda: _solve(kamsta, ctx, d, md, n, "boruvka_dev", kamsta.AlgorithmConfig())
+    ctx.set_memory_limit(_least_limit(kamsta, op) + (8 << 20))  # and the solves' vertex arrays
+    for _ in range(3):
+        solve()
+    assert _from_the_heap(kamsta, ctx, solve)
+    op(ctx)
+    torch.cuda.synchronize()
+    if what == "7bit":
+        ref, _ = oracle.kruskal(edges, n)
+        k = ctx.boruvka_7bit_dev(g, out.data_ptr())
+        got = out[:k].cpu().numpy().view(np.uint32).reshape(-1).view(kamsta.WEDGE)
+        assert np.array_equal(oracle.canon_keys(got), oracle.canon_keys(ref))
+    ctx.close()
+    gen.close()
