@@ -556,6 +556,7 @@ kamsta_status kamsta_ctx_trim(kamsta_ctx* ctx) {
   ctx->io.release();
   heap_release(ctx);
   ctx->heap.want = 0;
+  ctx->heap.too_large = ~0ull;
   if (ctx->pool) {
     cudaStreamSynchronize(ctx->stream);
     cudaMemPoolTrimTo(ctx->pool, 0);
@@ -570,7 +571,7 @@ kamsta_status kamsta_ctx_set_memory_limit(kamsta_ctx* ctx, uint64_t bytes) {
   }
   std::lock_guard<std::mutex> lock(ctx->mu);
   ctx->mem_limit = bytes;
-  ctx->heap.off = false;
+  ctx->heap.too_large = ~0ull;
   if (bytes && ctx_device_bytes(ctx) > bytes) {  // what only serves speed goes first
     heap_release(ctx);
     ctx->heap.want = 0;

@@ -915,9 +915,9 @@ kamsta_status solve_wave(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint3
     if (s == KAMSTA_OK) scope.finished();
     return s;
   };
-  kamsta_status s = once();
-  if (s == KAMSTA_E_OOM && heap_retry(ctx)) s = once();
-  return s;
+  uint64_t bytes = 0;
+  for (uint32_t i = 0; i < G; ++i) bytes += batch_graph_bytes(g[i].m_directed, g[i].n);
+  return heap_call(ctx, bytes, [&](bool) { return once(); });
 }
 
 // Autotuner of the batch path: times the persistent small-graph kernel at

@@ -59,6 +59,10 @@ struct kamsta_server {
     return std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0)
         .count();
   }
+  // Scratch for the common waves before the first one: growing the heap wave by
+  // wave stalls the workers (16 000 requests/s of the bench's mix, p99 24 ms
+  // grown so, 8.4 from the start; a third leaves room for arenas and pool).
+  size_t preset_heap() const { return static_cast<size_t>(worker_limit / 3); }
   void worker(int w);
 };
 
@@ -167,6 +171,8 @@ void kamsta_server::worker(int w) {
           if (s1 != KAMSTA_OK) d.status = s1;
           peak = std::max(peak, wave_peak_bytes(ctx));
         }
+        std::lock_guard<std::mutex> clk(ctx->mu);
+        ctx->heap.want = std::max(ctx->heap.want, preset_heap());
       }
       const double finish = now_us();
       std::lock_guard<std::mutex> lk(mu);
@@ -254,10 +260,7 @@ kamsta_status kamsta_server_create(int device, const kamsta_server_cfg* cfg,
     uint64_t keep = c.budget_bytes / c.workers;
     kamsta_ctx_set_memory_limit(ctx, keep);
     cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    // scratch for the common waves before the first one: growing the heap
-    // wave by wave stalls the workers (16 000 requests/s of the bench's mix,
-    // p99 24 ms grown so, 8.4 from the start; a third leaves room for arenas and pool)
-    ctx->heap.want = static_cast<size_t>(s->worker_limit / 3);
+    ctx->heap.want = s->preset_heap();
     {
       HeapScope heap(ctx, ctx->stream);
     }

@@ -122,14 +122,30 @@ static bool heap_give_back(kamsta_ctx* ctx) {
   return true;
 }
 
-// After a call that ran out of memory: gives the heap's block back and keeps
-// the context on its pool alone.  True when that can help (nothing of the
-// heap is in use and it held memory).
-bool heap_retry(kamsta_ctx* ctx) {
-  if (!heap_give_back(ctx)) return false;
-  ctx->heap.off = true;
-  ctx->heap.want = 0;
-  return true;
+// The next calls of that size run without a block at once, smaller ones keep
+// theirs.  A call that runs out of memory all the same says nothing about the
+// block, and neither it nor one that runs without sets its size.
+kamsta_status heap_call(kamsta_ctx* ctx, uint64_t bytes,
+                        const std::function<kamsta_status(bool)>& work) {
+  Heap& h = ctx->heap;
+  if (h.depth > 0) return work(false);  // the outermost call decides
+  const size_t want = h.want;
+  auto without = [&](bool again) -> kamsta_status {
+    h.off = true;
+    const kamsta_status s = work(again);
+    h.off = false;
+    h.want = want;
+    return s;
+  };
+  if (bytes >= h.too_large) {
+    heap_give_back(ctx);
+    return without(false);
+  }
+  kamsta_status s = work(false);
+  if (s != KAMSTA_E_OOM) return s;
+  h.want = want;
+  if (heap_give_back(ctx) && (s = without(true)) == KAMSTA_OK) h.too_large = bytes;
+  return s;
 }
 
 HeapScope::HeapScope(kamsta_ctx* ctx, cudaStream_t st) : ctx_(ctx), st_(st) {
@@ -2157,17 +2173,16 @@ kamsta_status solve_device(kamsta_ctx* ctx, Algo algo, const kamsta_wedge* d_in,
     if (r == KAMSTA_OK) scope.finished();
     return r;
   };
-  kamsta_status r = once();
-  if (r == KAMSTA_E_OOM && heap_retry(ctx)) {
-    // the heap holds memory that the limit (or the device) needs elsewhere
-    if (st) std::memset(st, 0, sizeof(*st));
-    if (d_forest_bits && cudaMemsetAsync(d_forest_bits, 0, ((m_directed + 31) / 32) * 4, str) !=
-                             cudaSuccess)
-      return r;
-    if (io) io->early = 0;
-    r = once();
-  }
-  return r;
+  return heap_call(ctx, 48 * m_directed + 96ull * n, [&](bool again) -> kamsta_status {
+    if (again) {
+      if (st) std::memset(st, 0, sizeof(*st));
+      if (d_forest_bits && cudaMemsetAsync(d_forest_bits, 0, ((m_directed + 31) / 32) * 4, str) !=
+                               cudaSuccess)
+        return KAMSTA_E_OOM;
+      if (io) io->early = 0;
+    }
+    return once();
+  });
 }
 
 }  // namespace kamsta

@@ -4,6 +4,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <utility>
@@ -60,7 +61,8 @@ struct Heap {
   std::vector<std::pair<void*, size_t>> pooled;  // this call's blocks from the pool
   cudaStream_t st = nullptr;       // the open call's stream
   int depth = 0;                   // > 0: open
-  bool off = false;                // a memory limit left no room for it
+  uint64_t too_large = ~0ull;      // calls of this size do not fit beside it
+  bool off = false;                // the open call runs without it (heap_call)
   void* take(size_t bytes);
   bool give(void* p);              // false: not from here
 };
@@ -229,7 +231,11 @@ class HeapScope {
   bool opened_ = false, synced_ = false;
 };
 void heap_release(kamsta_ctx* ctx);
-bool heap_retry(kamsta_ctx* ctx);
+// Runs a call's work; when it runs out of memory while the heap holds some, the
+// block is given back and the work (again = true) runs once more without one.
+// bytes: an estimate of the call's device memory, for telling calls apart.
+kamsta_status heap_call(kamsta_ctx* ctx, uint64_t bytes,
+                        const std::function<kamsta_status(bool again)>& work);
 cudaError_t ctx_reserve(kamsta_ctx* ctx, Arena& a, size_t bytes);
 
 }  // namespace kamsta

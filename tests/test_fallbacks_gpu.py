@@ -197,3 +197,44 @@ def test_idle_scratch_block_gives_way(kamsta, oracle, what, m_solve):
         assert np.array_equal(oracle.canon_keys(got), oracle.canon_keys(ref))
     ctx.close()
     gen.close()
+
+
+def test_out_of_memory_call_does_not_end_the_heap(kamsta):
+    """A call that ran out of memory, and one that fitted only without the
+    scratch block, leave later, smaller calls a block of scratch."""
+    import torch
+    n, cfg = 1 << 16, kamsta.AlgorithmConfig()
+    gen = kamsta.Context(0)
+    graphs = []
+    for m in (1 << 17, 1 << 20, 1 << 21, 1 << 23):
+        d = torch.empty((2 * m, 3), dtype=torch.int32, device="cuda")
+        graphs.append((d, gen.gen_gnm_dev(n, m, m, 254, d.data_ptr())))
+    want = [_solve(kamsta, gen, d, md, n, "boruvka_dev", cfg) for d, md in graphs]
+    ctx = kamsta.Context(0)
+
+    def solve(i):
+        d, md = graphs[i]
+        got = _solve(kamsta, ctx, d, md, n, "boruvka_dev", cfg)
+        assert np.array_equal(got, want[i])
+
+    d2, md2 = graphs[2]
+    ctx.set_memory_limit(_least_limit(
+        kamsta, lambda c: _solve(kamsta, c, d2, md2, n, "boruvka_dev", cfg)))
+    for _ in range(3):
+        solve(1)
+    assert _from_the_heap(kamsta, ctx, lambda: solve(1))
+    with pytest.raises(kamsta.KamstaError) as ei:
+        solve(3)                       # too large for the limit
+    assert ei.value.status == kamsta._native.E_OOM
+    solve(1)
+    assert _from_the_heap(kamsta, ctx, lambda: solve(1))
+    for _ in range(6):                 # fits, but not beside the block
+        solve(2)
+        solve(0)
+        assert _from_the_heap(kamsta, ctx, lambda: solve(0))
+    ctx.trim()
+    for _ in range(3):
+        solve(1)
+    assert _from_the_heap(kamsta, ctx, lambda: solve(1))
+    ctx.close()
+    gen.close()
