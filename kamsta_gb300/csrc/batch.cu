@@ -568,11 +568,12 @@ kamsta_status launch_small(kamsta_ctx* ctx, kamsta_graph_desc* g, const std::vec
     least += slot[c] + 4096;
   }
   if (ctx->mem_limit) {
-    // under a memory limit, only as many scratch slots as the limit leaves
-    // room for (one per class at least); the work queues spread the graphs
-    // over however many CTAs run
+    // under a memory limit, only as many scratch slots as the limit (or the
+    // heap, when it is this call's alone) leaves room for, one per class at
+    // least; the work queues spread the graphs over however many CTAs run
     const uint64_t used = ctx_device_bytes(ctx);
-    room = ctx->mem_limit > used ? ctx->mem_limit - used : 0;
+    room = std::max<uint64_t>(ctx->mem_limit > used ? ctx->mem_limit - used : 0,
+                              ctx->heap.room(st));
     room = room > least ? room - least : 0;
     for (int c = 0; c < kClasses; ++c) {
       if (!count[c]) continue;
@@ -821,15 +822,21 @@ kamsta_status solve_union(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint
 bool is_small_graph(const kamsta_ctx* ctx, const kamsta_graph_desc& g) { return is_small(ctx, g); }
 
 // Small graphs under way on the context's side streams.  A call that fails
-// midway waits for them: they use scratch that is freed in aux's order, which
-// the size classes' streams may not have joined yet, and the caller's buffers.
+// midway waits for them: they use scratch that is freed in their common
+// stream's order, which the size classes' streams may not have joined yet, and
+// the caller's buffers.  Alone on the wave's stream they use the heap as it is:
+// their slots adapt to the room there is and do not set its size.
 struct SmallInFlight {
   kamsta_ctx* ctx;
+  cudaStream_t on;
+  bool alone;
+  size_t want = ctx->heap.want;
   bool done = false;
   ~SmallInFlight() {
+    if (alone) ctx->heap.want = want;
     if (done) return;
     for (cudaStream_t s : ctx->small_st) cudaStreamSynchronize(s);
-    cudaStreamSynchronize(ctx->aux);
+    cudaStreamSynchronize(on);
   }
 };
 
@@ -841,14 +848,18 @@ static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_de
     ((!host_buffers && is_small(ctx, g[i])) ? sm : lg).push_back(i);
   if (sm.empty()) return solve_union(ctx, algo, g, G, cfg, host_buffers, st, ws);
   // small graphs on the auxiliary stream, overlapping the union solve (the
-  // forest is the same for boruvka and filter_boruvka)
-  B_TRY(cudaEventRecord(ctx->ev_fork, st));
-  B_TRY(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
+  // forest is the same for boruvka and filter_boruvka); without one on the
+  // wave's own, where their scratch comes from the heap
+  const cudaStream_t on = lg.empty() ? st : ctx->aux;
+  if (on != st) {
+    B_TRY(cudaEventRecord(ctx->ev_fork, st));
+    B_TRY(cudaStreamWaitEvent(on, ctx->ev_fork, 0));
+  }
   PoolBuf tab, scr;
-  SmallInFlight under_way{ctx};
+  SmallInFlight under_way{ctx, on, on == st};
   small::Result* d_res = nullptr;
   uint32_t launches = 0;
-  B_KTRY(launch_small(ctx, g, sm, cfg, false, ctx->aux, &tab, &scr, &d_res, &launches));
+  B_KTRY(launch_small(ctx, g, sm, cfg, false, on, &tab, &scr, &d_res, &launches));
   BatchWaveStats us;
   kamsta_status s = KAMSTA_OK;
   if (!lg.empty()) {
@@ -862,10 +873,12 @@ static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_de
   // after the union solve's launches)
   std::vector<small::Result> h_res(sm.size());
   B_TRY(cudaMemcpyAsync(h_res.data(), d_res, sizeof(small::Result) * sm.size(),
-                        cudaMemcpyDeviceToHost, ctx->aux));
-  B_TRY(cudaEventRecord(ctx->ev_join, ctx->aux));
-  B_TRY(cudaStreamWaitEvent(st, ctx->ev_join, 0));
-  B_TRY(cudaStreamSynchronize(ctx->aux));
+                        cudaMemcpyDeviceToHost, on));
+  if (on != st) {
+    B_TRY(cudaEventRecord(ctx->ev_join, on));
+    B_TRY(cudaStreamWaitEvent(st, ctx->ev_join, 0));
+  }
+  B_TRY(cudaStreamSynchronize(on));
   if (s != KAMSTA_OK) return s;
   uint64_t entries = 0, verts = 0;
   auto report = [](kamsta_graph_desc& d, const small::Result& r) {
@@ -890,11 +903,11 @@ static kamsta_status solve_wave_once(kamsta_ctx* ctx, Algo algo, kamsta_graph_de
   if (!again.empty()) {
     // edges listed in one direction only can be more than a class's lists
     // hold: those graphs once more in the largest class
-    B_KTRY(launch_small(ctx, g, again, cfg, true, ctx->aux, &tab, &scr, &d_res, &launches));
+    B_KTRY(launch_small(ctx, g, again, cfg, true, on, &tab, &scr, &d_res, &launches));
     h_res.resize(again.size());
     B_TRY(cudaMemcpyAsync(h_res.data(), d_res, sizeof(small::Result) * again.size(),
-                          cudaMemcpyDeviceToHost, ctx->aux));
-    B_TRY(cudaStreamSynchronize(ctx->aux));
+                          cudaMemcpyDeviceToHost, on));
+    B_TRY(cudaStreamSynchronize(on));
     for (size_t k = 0; k < again.size(); ++k) report(g[again[k]], h_res[k]);
   }
   under_way.done = true;

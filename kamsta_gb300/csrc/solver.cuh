@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 #include <functional>
@@ -65,6 +66,12 @@ struct Heap {
   bool off = false;                // the open call runs without it (heap_call)
   void* take(size_t bytes);
   bool give(void* p);              // false: not from here
+  size_t room(cudaStream_t on) const {  // largest block for the open call's stream
+    size_t most = 0;
+    if (depth > 0 && on == st)
+      for (const Region& r : free_list) most = std::max(most, r.size);
+    return most;
+  }
 };
 
 // Per-kernel counter block in device memory (zeroed before each round).

@@ -238,3 +238,35 @@ def test_out_of_memory_call_does_not_end_the_heap(kamsta):
     assert _from_the_heap(kamsta, ctx, lambda: solve(1))
     ctx.close()
     gen.close()
+
+
+def test_small_graphs_use_the_idle_scratch_block(kamsta, oracle):
+    """A wave of small graphs alone takes its slots from a block that a larger
+    wave left, also under a memory limit that the block nearly fills."""
+    import torch
+    ctx = kamsta.Context(0)
+    big = torch.empty((1 << 22, 3), dtype=torch.int32, device="cuda")
+    md = ctx.gen_gnm_dev(1 << 16, 1 << 21, 21, 254, big.data_ptr())
+    e, n = oracle.gen_gnm(3000, 20000, 22), 3000
+    ref = _sorted_forest(oracle, e, n)
+    d = _dev(e)
+    out = torch.zeros((65, 1 << 16, 3), dtype=torch.int32, device="cuda")
+    descs = (kamsta.GraphDesc * 65)()
+    for k in range(65):
+        descs[k].edges, descs[k].m_directed, descs[k].n = d.data_ptr(), len(e), n
+        descs[k].out = out[k].data_ptr()
+    descs[64].edges, descs[64].m_directed, descs[64].n = big.data_ptr(), md, 1 << 16
+    torch.cuda.synchronize()
+    large, small = (kamsta.GraphDesc * 1)(descs[64]), (kamsta.GraphDesc * 64)(*descs[:64])
+    for limit in (0, _least_limit(kamsta, lambda c: c.batch_dev(large)) + (1 << 20)):
+        ctx.set_memory_limit(limit)
+        for _ in range(3):
+            ctx.batch_dev(large)
+        out.zero_()
+        torch.cuda.synchronize()
+        assert _from_the_heap(kamsta, ctx, lambda: ctx.batch_dev(small))
+        assert all(g.status == 0 and g.out_count == len(ref) for g in small)
+        got = out[63, :len(ref)].cpu().numpy().view(np.uint32).reshape(-1).view(kamsta.WEDGE)
+        assert np.array_equal(got, ref)
+        assert _from_the_heap(kamsta, ctx, lambda: ctx.batch_dev(large))
+    ctx.close()
