@@ -574,6 +574,10 @@ kamsta_status launch_small(kamsta_ctx* ctx, kamsta_graph_desc* g, const std::vec
     const uint64_t used = ctx_device_bytes(ctx);
     room = std::max<uint64_t>(ctx->mem_limit > used ? ctx->mem_limit - used : 0,
                               ctx->heap.room(st));
+    // no room for one of each: one class after the other would do, and the
+    // largest takes them all
+    if (room < least && count[kClasses - 1] < S)
+      return launch_small(ctx, g, idx, cfg, true, st, tab, scr, d_res, launches);
     room = room > least ? room - least : 0;
     for (int c = 0; c < kClasses; ++c) {
       if (!count[c]) continue;

@@ -270,3 +270,26 @@ def test_small_graphs_use_the_idle_scratch_block(kamsta, oracle):
         assert np.array_equal(got, ref)
         assert _from_the_heap(kamsta, ctx, lambda: ctx.batch_dev(large))
     ctx.close()
+
+
+def test_small_graphs_of_all_classes_in_one_slot(kamsta, oracle):
+    """A memory limit with room for the largest class's slot (4.7 MB) but not
+    for one of each class (6.1 MB)."""
+    import torch
+    specs = [(500, 3000), (3000, 20000), (20000, 90000)]
+    graphs = [(oracle.gen_gnm(n, m, 31 + n), n) for n, m in specs]
+    dev = [_dev(e) for e, _ in graphs]
+    outs = [torch.zeros((n, 3), dtype=torch.int32, device="cuda") for _, n in graphs]
+    descs = (kamsta.GraphDesc * 3)()
+    for d, t, o, (e, n) in zip(descs, dev, outs, graphs):
+        d.edges, d.m_directed, d.n, d.out = t.data_ptr(), len(e), n, o.data_ptr()
+    torch.cuda.synchronize()
+    ctx = kamsta.Context(0)
+    ctx.set_memory_limit(5500000)
+    for _ in range(2):
+        ctx.batch_dev(descs)
+        for d, o, (e, n) in zip(descs, outs, graphs):
+            ref = _sorted_forest(oracle, e, n)
+            got = o[:len(ref)].cpu().numpy().view(np.uint32).reshape(-1).view(kamsta.WEDGE)
+            assert d.status == 0 and d.out_count == len(ref) and np.array_equal(got, ref)
+    ctx.close()
