@@ -1465,7 +1465,14 @@ cudaError_t launch_in_order(int dev, const void* f, uint32_t grid, uint32_t bloc
 // 575 / 183, 2^24 1272 / 859 (G(n,m), no preprocessing) and 1383 / 486 (RGG,
 // local preprocessing).  From 2^25 on the heaviest class is better contracted
 // by row scans than by the stream used here (2^26: 400 MB of reads).
+// With few entries the vertices are the work, and one CTA per SM streams them
+// slower than the host-driven kernels once they fill those.  G(n,m) without
+// preprocessing, host-driven against cooperative: n = 2^22, n / m = 4, 1/2: 270
+// / 238, 895 / 869; 2^23: 404 / 376, 1660 / 1630; 2^24, n / m = 16, 4, 1: 491 /
+// 461, 677 / 663, 1601 / 1647; 2^25, n / m = 16, 4, 2: 855 / 860, 1276 / 1348,
+// 1967 / 2054; 2^26, n / m = 16, 4: 1549 / 1632, 2696 / 2842.
 constexpr uint64_t kCoopMaxMd = (1ull << 25) - 1;
+constexpr uint32_t kCoopMaxN = 1u << 24;
 
 bool Solve::coop_options() const {
   // per-round traces, dedupe between rounds and the debug checks are the
@@ -1477,7 +1484,8 @@ bool Solve::coop_options() const {
 }
 
 bool Solve::coop_fits() const {
-  return coop_now() && !uni_ && md_ <= kCoopMaxMd && bounds_.size() + 1 <= coop::kMaxLaunch;
+  return coop_now() && !uni_ && md_ <= kCoopMaxMd && n_ <= kCoopMaxN &&
+         bounds_.size() + 1 <= coop::kMaxLaunch;
 }
 
 // One CTA per SM; little work takes fewer, so that its barriers are short.

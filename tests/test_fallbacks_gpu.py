@@ -293,3 +293,28 @@ def test_small_graphs_of_all_classes_in_one_slot(kamsta, oracle):
             got = o[:len(ref)].cpu().numpy().view(np.uint32).reshape(-1).view(kamsta.WEDGE)
             assert d.status == 0 and d.out_count == len(ref) and np.array_equal(got, ref)
     ctx.close()
+
+
+@pytest.mark.parametrize("n,cooperative", [(1 << 24, True), ((1 << 24) + 1, False)])
+@pytest.mark.parametrize("lp", [0, 1])
+def test_sparse_graphs_at_the_vertex_limit(kamsta, n, cooperative, lp):
+    """Few edges on many vertices: cooperative rounds up to 2^24 vertices,
+    host-driven ones beyond, the forest byte for byte that of a traced solve."""
+    import torch
+    ctx = kamsta.Context(0)
+    d = torch.empty((1 << 22, 3), dtype=torch.int32, device="cuda")
+    md = ctx.gen_gnm_dev(n, 1 << 21, 41, 254, d.data_ptr())
+    o = torch.zeros((2, n, 3), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    want, got = {}, {}
+    kw = ctx.boruvka_dev(d.data_ptr(), md, n, o[0].data_ptr(),
+                         kamsta.AlgorithmConfig(local_preprocessing=lp, trace=True), stats=want)
+    _fail(kamsta, ctx, COOP_LAUNCH, 1000)
+    k = ctx.boruvka_dev(d.data_ptr(), md, n, o[1].data_ptr(),
+                        kamsta.AlgorithmConfig(local_preprocessing=lp), stats=got)
+    launches = 1000 - _fail(kamsta, ctx, COOP_LAUNCH, 0)
+    assert (got["phases"]["round_verts"]["launches"] == 0) == cooperative
+    assert launches == 1 or not cooperative
+    assert k == kw and got["total_weight"] == want["total_weight"]
+    assert torch.equal(o[0], o[1])
+    ctx.close()
