@@ -196,7 +196,8 @@ kamsta_status kamsta_mst_boruvka_wedge64(const kamsta_wedge64* edges,
 
 /* ---- single-graph solve, device buffers --------------------------------
  * d_edges / d_out are device pointers; the call is stream-ordered on
- * `stream` and returns after the result count is known.  out_count and stats are host pointers.                   */
+ * `stream` and returns after the result count is known.  out_count and stats
+ * are host pointers. */
 kamsta_status kamsta_mst_boruvka_dev(kamsta_ctx* ctx, const kamsta_wedge* d_edges,
                                      uint64_t m_directed, uint32_t n,
                                      const kamsta_cfg* cfg, kamsta_wedge* d_out,
@@ -327,7 +328,8 @@ kamsta_status kamsta_ctx_set_tiles(kamsta_ctx* ctx, uint32_t items_per_thread,
 typedef struct kamsta_server kamsta_server;
 
 typedef struct kamsta_server_cfg {
-  uint64_t budget_bytes;     /* admission budget, device bytes (0 = 64 GiB)   */
+  uint64_t budget_bytes;     /* admission budget, device bytes (0 = 64 GiB);  */
+                             /* three eighths of it are allocated at creation */
   uint32_t max_batch;        /* jobs per wave at most (0 = 4096)              */
   uint32_t workers;          /* worker threads / streams (1..8, default 2)   */
   kamsta_cfg solver;         /* solver options for every job (FILTER flag    */

@@ -39,9 +39,10 @@ std::vector<std::pair<uint32_t, uint32_t>> plan_waves(const kamsta_graph_desc* g
                                                       uint64_t budget);
 
 // One wave.  Small graphs (n <= 32768, m_directed <= 262144; device
-// buffers only) go to one persistent launch on the context's auxiliary
-// stream, one CTA per graph from a work queue; the others are solved as
-// their disjoint union on `st`, the forest split back per graph.  Either
+// buffers only) go to persistent launches on the context's side streams (from
+// `st` itself in a wave of small graphs alone), one CTA per graph from a work
+// queue; the others are solved as their disjoint union on `st`, the forest
+// split back per graph.  Either
 // way each forest is sorted by (src, dst).  host_buffers: edges/out are host
 // pointers.
 kamsta_status solve_wave(kamsta_ctx* ctx, Algo algo, kamsta_graph_desc* g, uint32_t G,

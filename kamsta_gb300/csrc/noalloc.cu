@@ -4,10 +4,9 @@
 // framework's fixed memory budget, an allocator-less runtime, or a plugin
 // that is handed a stream and buffers and must not touch the device heap.
 // kamsta_mst_boruvka_noalloc serves them: it runs the Boruvka rounds of
-// kamsta_mst_boruvka_dev (hook, pointer jumping, renumbering, relabel +
-// self-loop removal + stable compaction) fused into one single-CTA kernel
-// (small_solve.cuh), and every scratch byte it needs lives in the file-scope
-// array below.
+// kamsta_mst_boruvka_dev (hook, renumbering, label walk, relabel + self-loop
+// removal) fused into one single-CTA kernel (small_solve.cuh), and every
+// scratch byte it needs lives in the file-scope array below.
 //
 // Limits: n <= kNoallocMaxN vertices and m_directed <= kNoallocMaxMd input
 // entries.  The array (about 5 MB) is part of the library image, so every

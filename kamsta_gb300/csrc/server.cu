@@ -118,7 +118,7 @@ void kamsta_server::worker(int w) {
       more = !queue.empty();
     }
     if (more) cv_work.notify_one();  // more work for another worker
-    // small jobs first (one persistent launch, finished in well under a
+    // small jobs first (persistent launches, finished in well under a
     // millisecond), then the rest as one union solve; each group completes
     // as soon as it is done
     std::stable_partition(batch.begin(), batch.end(), [ctx](const Job& j) {

@@ -752,6 +752,9 @@ kamsta_status Solve::pass(int phase, const SegList* src, const uint32_t* map, ui
   const size_t dyn = dir ? dir_dyn_smem(items)
                          : rec_dyn_smem(sitems) + round_up(size_t(smin_n) * 8, 16);
   const bool mapped = map != nullptr;
+  // (the variant is built for the default tile alone, and long rows are looked
+  // for in the sample that the plan of weight classes draws: plain rounds have
+  // none, and one costs a small call a fifth of its time)
   const bool hub = dir && !mapped && items == 6 && long_rows_ && direct_emit_;
   const bool uni = dir && uni_ != nullptr;
   static_assert(kUnionMinGraph > dir_tile(kItemsDir) + 4, "a tile lies in two graphs at most");

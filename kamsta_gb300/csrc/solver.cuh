@@ -48,7 +48,7 @@ struct Arena {
 // room so that it grows rarely.  It comes from the pool, which still holds what
 // the call before had taken there (a context's second call on G(n,m)
 // 2^26/2^30: 39.0 ms with a block of its own memory, 21.6 so; later ones
-// 20.1).
+// 20.1).  The first call has none: nothing says how large it should be.
 struct Heap {
   struct Region {
     size_t off, size;
